@@ -159,18 +159,15 @@ typedef struct pm_ctx pm_ctx;
  * to tune. */
 #define PM_STAGING_MAX 64
 typedef struct pm_tuning {
-  int variant;          /* FP32 kernel of the one-warp grids: 0 = 168 registers per thread (3 blocks of 4
-                           warps per SM), 1 = 128 (4 blocks per SM, a few spills), 2 = lock-step blocks
-                           (128 registers; the warps of a block run each LM pass together, so they share
-                           the instruction-cache lines of its parts; nine or ten free parameters without a
-                           v_mac row, one-warp grids; elsewhere 2 runs as 1) */
+  int variant;          /* 0, 1 or 2: one FP32 kernel serves the one-warp grids whatever it says; kept for
+                           hosts that set it, with the block sizes that go with each value */
   int staging_depth;    /* host-buffer calls on grids of <= 32 wavelengths: the cube goes in at most
                            this many pieces, each twice the one before; one persistent launch inverts
                            them as the copy stream publishes each piece (1..PM_STAGING_MAX); 0 = copy
                            everything, then launch.  Output buffers in pinned, mapped host memory
                            (cudaHostAlloc) receive each pixel's results from the kernel directly */
-  int warps_per_block;  /* pixels (one warp each) per block of the one-warp kernels: 1, 2 or 4; with
-                           variant 2: 4, 8 or 16 */
+  int warps_per_block;  /* warps per block of the one-warp kernels (FP32 triplets: two pixels per warp,
+                           otherwise one): 1, 2 or 4; with variant 2: 4, 8 or 16, run as 4 */
   int graphs;           /* 1: host-buffer calls of at most PM_GRAPH_MAX_PIXELS pixels on grids of <= 32
                            wavelengths (pm_lm_mils among them) stage through pinned memory and replay a
                            CUDA graph of the whole call, captured once per size; 0: no graphs */

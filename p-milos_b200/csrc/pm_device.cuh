@@ -81,6 +81,12 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// A condition that has the same value in every lane, as a vote: the compiler then
+// sees a branch that the warp takes as one.  Behind a branch it takes for a
+// divergent one, every shuffle and warp barrier costs extra instructions (the
+// normal equations' code was twice as long).
+__device__ __forceinline__ bool uniform(bool c) { return __any_sync(kFull, c); }
+
 // ---------------------------------------------------------------------------
 // Voigt / Faraday-Voigt: H = Re w, F = Im w / 2 (fvoigt.c:15-80).  Horner in
 // complex arithmetic, then a branch-free Smith (1962) division.
@@ -229,6 +235,41 @@ struct alignas(16) LaneState {
 static_assert(sizeof(LaneState<float>) == kLaneStatePad * sizeof(float), "LaneState layout");
 static_assert(sizeof(LaneState<double>) == kLaneStatePad * sizeof(double), "LaneState layout");
 
+// The propagation matrix of the groups' profiles s.fi and s.shi and the
+// Unno-Rachkovsky solution (mil_sinrf.c:181-285).
+template <typename R>
+__device__ __forceinline__ void propagate(const ModelTerms<R>& T, LaneState<R>& s, R S[4]) {
+  s.parcial1 = s.fi[1] + s.fi[2];
+  s.parcial2 = T.E0_2 * (s.fi[0] - s.parcial1 / R(2));
+  s.parcial3 = T.E0_2 * (s.shi[0] - (s.shi[1] + s.shi[2]) / R(2));
+  s.etain = T.E0_2 * (s.fi[0] * T.sinis + s.parcial1 * T.cosis_2);
+  s.etaq = s.parcial2 * T.sinis_cosa;
+  s.etau = s.parcial2 * T.sinis_sina;
+  s.etav = (s.fi[2] - s.fi[1]) * T.cosi_E0_2;
+  s.rhoq = s.parcial3 * T.sinis_cosa;
+  s.rhou = s.parcial3 * T.sinis_sina;
+  s.rhov = (s.shi[2] - s.shi[1]) * T.cosi_E0_2;
+  s.etai = R(1) + s.etain;
+  s.etai_2 = s.etai * s.etai;
+  const R auxq = s.rhoq * s.rhoq, auxu = s.rhou * s.rhou, auxv = s.rhov * s.rhov;
+  s.gp1 = s.etai_2 - s.etaq * s.etaq - s.etau * s.etau - s.etav * s.etav + auxq + auxu + auxv;
+  s.gp3 = s.etai_2 + auxq + auxu + auxv;
+  s.gp2 = s.etaq * s.rhoq + s.etau * s.rhou + s.etav * s.rhov;
+  s.dt = s.etai_2 * s.gp1 - s.gp2 * s.gp2;
+  s.dti = R(1) / s.dt;
+  const R gp4 = s.etai_2 * s.etaq + s.etai * (s.etav * s.rhou - s.etau * s.rhov);
+  const R gp5 = s.etai_2 * s.etau + s.etai * (s.etaq * s.rhov - s.etav * s.rhoq);
+  const R gp6 = s.etai_2 * s.etav + s.etai * (s.etau * s.rhoq - s.etaq * s.rhou);
+  s.g4 = gp4 + s.rhoq * s.gp2;
+  s.g5 = gp5 + s.rhou * s.gp2;
+  s.g6 = gp6 + s.rhov * s.gp2;
+  const R dtiaux = R(s.dti * T.B1);
+  S[0] = R(T.B0 - double(dtiaux * s.etai * s.gp3));
+  S[1] = dtiaux * s.g4;
+  S[2] = dtiaux * s.g5;
+  S[3] = dtiaux * s.g6;
+}
+
 // ME synthesis at wavelength offset dl (mil_sinrf.c:117-285): the three Zeeman
 // groups (funcionComponentFor_sinrf, mil_sinrf.c:418-449: the strength-weighted
 // sum of every component's Voigt and Faraday-Voigt profiles), the propagation
@@ -266,35 +307,7 @@ __device__ __forceinline__ void synth_lane(const PmParams& P, const ModelTerms<R
       s.F[g] = F;
     }
   }
-  s.parcial1 = s.fi[1] + s.fi[2];
-  s.parcial2 = T.E0_2 * (s.fi[0] - s.parcial1 / R(2));
-  s.parcial3 = T.E0_2 * (s.shi[0] - (s.shi[1] + s.shi[2]) / R(2));
-  s.etain = T.E0_2 * (s.fi[0] * T.sinis + s.parcial1 * T.cosis_2);
-  s.etaq = s.parcial2 * T.sinis_cosa;
-  s.etau = s.parcial2 * T.sinis_sina;
-  s.etav = (s.fi[2] - s.fi[1]) * T.cosi_E0_2;
-  s.rhoq = s.parcial3 * T.sinis_cosa;
-  s.rhou = s.parcial3 * T.sinis_sina;
-  s.rhov = (s.shi[2] - s.shi[1]) * T.cosi_E0_2;
-  s.etai = R(1) + s.etain;
-  s.etai_2 = s.etai * s.etai;
-  const R auxq = s.rhoq * s.rhoq, auxu = s.rhou * s.rhou, auxv = s.rhov * s.rhov;
-  s.gp1 = s.etai_2 - s.etaq * s.etaq - s.etau * s.etau - s.etav * s.etav + auxq + auxu + auxv;
-  s.gp3 = s.etai_2 + auxq + auxu + auxv;
-  s.gp2 = s.etaq * s.rhoq + s.etau * s.rhou + s.etav * s.rhov;
-  s.dt = s.etai_2 * s.gp1 - s.gp2 * s.gp2;
-  s.dti = R(1) / s.dt;
-  const R gp4 = s.etai_2 * s.etaq + s.etai * (s.etav * s.rhou - s.etau * s.rhov);
-  const R gp5 = s.etai_2 * s.etau + s.etai * (s.etaq * s.rhov - s.etav * s.rhoq);
-  const R gp6 = s.etai_2 * s.etav + s.etai * (s.etau * s.rhoq - s.etaq * s.rhou);
-  s.g4 = gp4 + s.rhoq * s.gp2;
-  s.g5 = gp5 + s.rhou * s.gp2;
-  s.g6 = gp6 + s.rhov * s.gp2;
-  const R dtiaux = R(s.dti * T.B1);
-  S[0] = R(T.B0 - double(dtiaux * s.etai * s.gp3));
-  S[1] = dtiaux * s.g4;
-  S[2] = dtiaux * s.g5;
-  S[3] = dtiaux * s.g6;
+  propagate<R>(T, s, S);
 }
 
 // Shared memory.  Per block: the PSF taps, centred and reversed, in VEC shifted
@@ -338,9 +351,6 @@ struct alignas(16) WarpSmem {
   long long job_k;
   int grid_cur;
   int xs_dirty;  // xs holds macroturbulence data: restore its zero padding before psf_rows
-  // the lock-step kernel's ticket state: the last published count seen and the
-  // first ticket and pixel count of `job`
-  unsigned long long avail_seen, job_t0, job_n;
   unsigned long long pad_;
 };
 
@@ -490,8 +500,8 @@ __device__ __forceinline__ void mac_triple(const PmParams& P, double k, int lane
 }
 
 // The kernel of v_mac (and its derivative with DERIV) into xs; tr is scratch.
-template <typename R, bool DERIV>
-__device__ __forceinline__ void mac_prepare(const PmParams& P, WarpSmem<R>& sm, double mac, double dl, int lane,
+template <typename R, bool DERIV, typename SM>
+__device__ __forceinline__ void mac_prepare(const PmParams& P, SM& sm, double mac, double dl, int lane,
                                             bool valid) {
   double g, gd;
   mac_kernel<DERIV>(P, mac, dl, lane, valid, reinterpret_cast<double*>(sm.tr), g, gd);
@@ -520,10 +530,10 @@ __device__ __forceinline__ void mac_circular4(const PmParams& P, const R* xf, co
 
 // The 32 response-function profiles (one per lane, rows of tr) convolved
 // circularly with the kernel in xs, in place.
-template <typename R>
-__device__ __forceinline__ void mac_rf_circular(const PmParams& P, WarpSmem<R>& sm, int lane) {
+template <typename R, int STRIDE = TRS, typename SM>
+__device__ __forceinline__ void mac_rf_circular(const PmParams& P, SM& sm, int lane) {
   __syncwarp();
-  R* row = sm.tr + lane * TRS;
+  R* row = sm.tr + lane * STRIDE;
   const R* k3 = &sm.xs[0][0] + kMacK + P.half + P.nl;
   R acc[NL];
 #pragma unroll
@@ -541,8 +551,8 @@ __device__ __forceinline__ void mac_rf_circular(const PmParams& P, WarpSmem<R>& 
 }
 
 // Zero the padded rows again after macroturbulence data.
-template <typename R>
-__device__ __forceinline__ void xs_restore(WarpSmem<R>& sm, int lane) {
+template <typename R, typename SM>
+__device__ __forceinline__ void xs_restore(SM& sm, int lane) {
   for (int e = lane; e < 4 * XSR; e += 32) (&sm.xs[0][0])[e] = R(0);
   __syncwarp();
   if (lane == 0) sm.xs_dirty = 0;
@@ -556,16 +566,14 @@ __device__ __forceinline__ void xs_restore(WarpSmem<R>& sm, int lane) {
 // leaves them in globals.  MAC: the kernel has a v_mac response row (NTERMS >=
 // 10), so v_mac may be nonzero.  dl: this lane's wavelength offset lambda -
 // lambda0 (the grid's, or the pixel's own).
-template <typename R, bool MAC = false, bool ZM = false>
-__device__ __forceinline__ void synthesize(const PmParams& P, WarpSmem<R>& sm, const double* m,
-                                           const float* sl_pix, int lane, bool valid, double dl, R S[4], R Su[4]) {
-  ModelTerms<R> T;
-  LaneState<R> st;
-  model_terms<R, ZM>(P, m, T);
-  synth_lane<R, ZM>(P, T, dl, st, S);
-  copy16(*reinterpret_cast<LaneState<R>*>(sm.ls[lane]), st);
-  if (lane == 0) copy16(sm.mt, T);
-  const double mac = MAC ? m[9] : 0.0;
+template <typename R, bool MAC, bool SL, typename SM, typename Lane, typename Psf>
+__device__ __forceinline__ void synthesize_terms(const PmParams& P, SM& sm, const ModelTerms<R>& T, double mac,
+                                                 const float* sl_pix, int lane, bool valid, double dl, R S[4],
+                                                 R Su[4], Lane synth, Psf psf) {
+  R s0[4];
+  synth(s0);
+#pragma unroll
+  for (int s = 0; s < 4; ++s) S[s] = s0[s];
   if (MAC && mac > kMacMin) {
     R* xf = &sm.xs[0][0];
 #pragma unroll
@@ -578,11 +586,11 @@ __device__ __forceinline__ void synthesize(const PmParams& P, WarpSmem<R>& sm, c
     __syncwarp();
   } else if (P.has_psf) {
     if (MAC && sm.xs_dirty) xs_restore<R>(sm, lane);
-    psf_rows<R>(P, sm, lane, valid, S);
+    psf();
   }
 #pragma unroll
   for (int s = 0; s < 4; ++s) Su[s] = S[s];
-  if (P.slight_mode != PM_SLIGHT_NONE) {
+  if (SL && P.slight_mode != PM_SLIGHT_NONE) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
       const int idx = s * P.nl + (valid ? lane : 0);
@@ -591,6 +599,19 @@ __device__ __forceinline__ void synthesize(const PmParams& P, WarpSmem<R>& sm, c
     }
   }
   __syncwarp();
+}
+
+template <typename R, bool MAC = false, bool ZM = false>
+__device__ __forceinline__ void synthesize(const PmParams& P, WarpSmem<R>& sm, const double* m,
+                                           const float* sl_pix, int lane, bool valid, double dl, R S[4], R Su[4]) {
+  ModelTerms<R> T;
+  model_terms<R, ZM>(P, m, T);
+  synthesize_terms<R, MAC, true>(P, sm, T, MAC ? m[9] : 0.0, sl_pix, lane, valid, dl, S, Su, [&](R(&out)[4]) {
+    LaneState<R> st;
+    synth_lane<R, ZM>(P, T, dl, st, out);
+    copy16(*reinterpret_cast<LaneState<R>*>(sm.ls[lane]), st);
+    if (lane == 0) copy16(sm.mt, T);
+  }, [&] { psf_rows<R>(P, sm, lane, valid, S); });
 }
 
 template <typename R>
@@ -704,8 +725,7 @@ __device__ __forceinline__ void rf_lane(const PmParams& P, const ModelTerms<R>& 
 // row and the 32 taps of all outputs as aligned broadcast vector loads.  FP32
 // takes the inputs four at a time: their taps are one window of 35 consecutive
 // entries of a reversed tap row (9 vector loads for 128 products instead of 32),
-// which matters because all warps of a lock-step block run this loop together and
-// the broadcast loads were bound by shared-memory bandwidth; every output still
+// which the loop was bound by; every output still
 // adds its products in the order of m, so the results are those of the one-input
 // loop bit for bit.  Stokes-I rows correlate Ic - x with Ic = max of the row's end
 // points.
@@ -1513,214 +1533,6 @@ __device__ __forceinline__ void invert_pixel(const PmParams& P, const BlockSmem<
   if (spectra && valid) {
 #pragma unroll
     for (int s = 0; s < 4; ++s) spectra[base + s * P.nl + lane] = float(S[s]);
-  }
-  __syncwarp();
-}
-
-// ---------------------------------------------------------------------------
-// lm_mils in phases, for kernels whose warps advance in lock-step: the state of
-// one pixel's LM loop lives in registers (PixelLM) between three phases that a
-// block runs together, separated by block barriers -- the damped solve, the
-// synthesis with chi^2 and the acceptance test, the response functions with the
-// normal equations (accepted steps) -- so that at any time every warp of the
-// block executes the same phase's code.  Per pixel the arithmetic and its order
-// are those of invert_pixel.
-// ---------------------------------------------------------------------------
-template <typename R>
-struct PixelLM {
-  float O[4];
-  R isig[4];
-  R S[4], Su[4];
-  const float* sl_pix;
-  double dlp;
-  double ochi, chi0, chi, flambda, factor;
-  int nfree, status, iter, accepted, fallbacks;
-  bool stop, first, accept, finished;
-};
-
-// Before the loop (invert_pixel up to its first pass): the pixel's profiles,
-// ghosts, starting model; finished at once when nfree == 0.
-template <typename R, bool PIXGRID>
-__device__ __forceinline__ void lm_begin(const PmParams& P, const BlockSmem<R>& bs, WarpSmem<R>& sm, int lane,
-                                         PixelLM<R>& L) {
-  const bool valid = lane < P.nl;
-  double* m = sm.model;
-  const PmJob* jp = sm.job;
-  const size_t p = sm.pix;
-  const size_t base = p * 4 * P.nl;
-  L.sl_pix = slight_of<R>(P, bs, P.slight_mode == PM_SLIGHT_PER_PIXEL ? ld_ptr(&jp->slight) : nullptr, base);
-  const float* obs = ld_ptr(&jp->spectro) + base;
-  const double* model_in = ld_ptr(&jp->model_in);
-  L.dlp = 0.0;
-  if constexpr (PIXGRID) L.dlp = valid ? __ldcg(ld_ptr(&jp->lambda) + p * P.nl + lane) - P.lambda0 : 0.0;
-  const double dl = PIXGRID ? L.dlp : P.dl[valid ? lane : 0];
-  int ghosts = 0;
-  if ((reinterpret_cast<uintptr_t>(obs) & 15) == 0) {
-    // the pixel's 4 x nl floats as nl 16-byte loads (one per lane, one
-    // instruction for the warp), redistributed to lane = wavelength through the
-    // warp's transpose buffer (idle while a pixel starts)
-    float* stage = reinterpret_cast<float*>(sm.tr);
-    if (lane < P.nl) reinterpret_cast<float4*>(stage)[lane] = __ldcg(reinterpret_cast<const float4*>(obs) + lane);
-    __syncwarp();
-#pragma unroll
-    for (int s = 0; s < 4; ++s) L.O[s] = valid ? stage[s * P.nl + lane] : 0.0f;
-    __syncwarp();
-  } else {
-#pragma unroll
-    for (int s = 0; s < 4; ++s) L.O[s] = valid ? __ldcg(obs + s * P.nl + lane) : 0.0f;
-  }
-#pragma unroll
-  for (int s = 0; s < 4; ++s) {
-    const bool g = valid && L.O[s] <= -1.0f;
-    ghosts += __popc(__ballot_sync(kFull, g));
-    L.isig[s] = R(1.0 / (g ? kGhostSigma : P.noise));
-  }
-  if (model_in) {
-    if (lane < 11) m[lane] = __ldcg(model_in + p * 11 + lane);
-  } else {
-    double g[11];
-#pragma unroll
-    for (int i = 0; i < 11; ++i) g[i] = P.guess[i];
-    if (P.classical) classical(P, L.O, lane, valid, dl, g);
-    double mine = g[0];
-#pragma unroll
-    for (int i = 1; i < 11; ++i)
-      if (lane == i) mine = g[i];
-    if (lane < 11) m[lane] = mine;
-  }
-  __syncwarp();
-  L.nfree = P.nfree_base - ghosts;
-  L.status = PM_PIX_MAXITER;
-  L.iter = 0;
-  L.accepted = 0;
-  L.fallbacks = 0;
-  L.ochi = 0;
-  L.chi0 = 0;
-  L.chi = 0;
-  L.flambda = P.ilambda;
-  L.factor = 1.0;
-  L.stop = false;
-  L.first = true;
-  L.accept = false;
-  L.finished = false;
-  if (L.nfree == 0) {
-    L.status = PM_PIX_NFREE;
-    L.iter = -1;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) L.S[s] = 0;
-    L.finished = true;
-  } else {
-    if (lane < 11) sm.trial[lane] = m[lane];
-    __syncwarp();
-  }
-}
-
-// Phase 1: the damped solve and the trial model (every pass but the first).
-template <typename R, int KT>
-__device__ __forceinline__ void lm_solve(const PmParams& P, WarpSmem<R>& sm, int lane, PixelLM<R>& L) {
-  if (L.first) return;
-  double dlt[KT];
-  bool ok = true;
-  double* scratch = reinterpret_cast<double*>(sm.tr);
-  if (P.solver == PM_SOLVE_CHOLESKY) ok = solve_cholesky<KT>(sm.sv, scratch, lane, L.flambda, dlt);
-  if (P.solver != PM_SOLVE_CHOLESKY || !ok) {
-    if (P.solver == PM_SOLVE_CHOLESKY) ++L.fallbacks;
-    solve_eigen<KT>(sm.sv, scratch, lane, L.flambda);
-#pragma unroll
-    for (int i = 0; i < KT; ++i) dlt[i] = sm.sv.delta[i];
-    __syncwarp();
-  }
-  double t[11];
-#pragma unroll
-  for (int i = 0; i < 11; ++i) t[i] = sm.trial[i];
-  apply_delta<KT>(P, sm.model, dlt, t);
-  check_model(t);
-  __syncwarp();
-#pragma unroll
-  for (int i = 0; i < 11; ++i)
-    if (lane == i) sm.trial[i] = t[i];
-  __syncwarp();
-}
-
-// Phase 2: synthesis of the trial model, chi^2, the stopping and acceptance tests.
-template <typename R, bool MAC, bool PIXGRID, bool ZM>
-__device__ __forceinline__ void lm_synth(const PmParams& P, WarpSmem<R>& sm, int lane, PixelLM<R>& L) {
-  const bool valid = lane < P.nl;
-  const double dl = PIXGRID ? L.dlp : P.dl[valid ? lane : 0];
-  synthesize<R, MAC, ZM>(P, sm, sm.trial, L.sl_pix, lane, valid, dl, L.S, L.Su);
-  L.chi = chisq<R>(P, L.S, L.O, L.isig, valid, double(L.nfree));
-  L.accept = true;
-  if (!L.first) {
-    if ((fabs((L.ochi - L.chi) * 100 / L.chi) < P.toplim) || (L.chi < 0.0001)) {
-      L.stop = true;
-      L.status = PM_PIX_CONVERGED;
-    }
-    L.accept = L.chi - L.ochi < 0.;
-  }
-}
-
-// Phase 3: on acceptance the response functions and normal equations at the
-// new model; the damping update and the loop's end test.
-template <typename R, int KT, bool MAC, bool PIXGRID, bool ZM>
-__device__ __forceinline__ void lm_update(const PmParams& P, const BlockSmem<R>& bs, WarpSmem<R>& sm, int lane,
-                                          PixelLM<R>& L) {
-  const bool valid = lane < P.nl;
-  const double dl = PIXGRID ? L.dlp : P.dl[valid ? lane : 0];
-  if (L.accept) {
-    if (!L.first) L.flambda = L.flambda / (5.0 * L.factor);
-    if (lane < 11) sm.model[lane] = sm.trial[lane];
-    __syncwarp();
-    R Sff[4];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) Sff[s] = L.first ? L.Su[s] : L.S[s];
-    rf_and_normal_eq<R, KT, MAC, ZM>(P, bs, sm, lane, valid, dl, L.S, Sff, L.O, L.isig, L.sl_pix);
-    L.ochi = L.chi;
-    if (L.first) L.chi0 = L.chi;
-    else ++L.accepted;
-  } else {
-    L.flambda = L.flambda * 10.0 * L.factor;
-  }
-  if (!L.first) {
-    if ((L.flambda > 1e+7) || (L.flambda < 1e-25)) {
-      if (!L.stop) L.status = PM_PIX_LAMBDA;
-      L.stop = true;
-    }
-    ++L.iter;
-    if (P.logclambda) L.factor = double(log10f(float(L.chi)) / log10f(float(L.chi0)));
-    if (!(L.iter < P.miter && !L.stop)) L.finished = true;
-  }
-  L.first = false;
-}
-
-// After the loop: the finite check and the pixel's results (invert_pixel's outputs).
-template <typename R>
-__device__ __forceinline__ void lm_end(const PmParams& P, WarpSmem<R>& sm, int lane, PixelLM<R>& L,
-                                       unsigned long long* ctr) {
-  const bool valid = lane < P.nl;
-  double* m = sm.model;
-  if (L.nfree != 0) {
-    bool finite = isfinite(L.ochi);
-#pragma unroll
-    for (int i = 0; i < 11; ++i) finite = finite && isfinite(m[i]);
-    if (!finite) L.status = PM_PIX_NONFINITE;
-  }
-  const PmJob* jp = *reinterpret_cast<const PmJob* const volatile*>(&sm.job);
-  const size_t p = *reinterpret_cast<const volatile unsigned long long*>(&sm.pix);
-  const size_t base = p * 4 * P.nl;
-  if (lane < 11) ld_ptr(&jp->models)[p * 11 + lane] = m[lane];
-  if (lane == 0) {
-    ld_ptr(&jp->chisq)[p] = float(L.ochi);
-    ld_ptr(&jp->iters)[p] = L.iter;
-    int* st = ld_ptr(&jp->status);
-    if (st) st[p] = L.status;
-    atomicAdd(&ctr[PMC_ITERS], (unsigned long long)(L.iter > 0 ? L.iter : 0));
-    atomicAdd(&ctr[PMC_ACCEPTED], (unsigned long long)L.accepted);
-    if (L.fallbacks) atomicAdd(&ctr[PMC_FALLBACK], (unsigned long long)L.fallbacks);
-  }
-  float* spectra = ld_ptr(&jp->spectra);
-  if (spectra && valid) {
-#pragma unroll
-    for (int s = 0; s < 4; ++s) spectra[base + s * P.nl + lane] = float(L.S[s]);
   }
   __syncwarp();
 }

@@ -115,7 +115,7 @@ struct SmallStage {
 struct pm_ctx {
   PmParams P;
   int precision = PM_PREC_FP32;
-  pm_tuning tuning{2, 8, 16, 1};  // lock-step blocks of 16 warps (FP32 one-warp grids), fed in up to 8 pieces
+  pm_tuning tuning{2, 8, 16, 1};  // host-buffer calls fed in up to 8 pieces, small ones as graphs
   int device = 0;
   int num_sms = 148;
   cudaStream_t stream = nullptr;
@@ -303,11 +303,15 @@ int fill_params(const pm_line* L, const pm_config* c, PmParams& P) {
   P.solver = solver;
   P.n_pi = L->n_pi;
   P.n_sig = L->n_sig;
-  for (int i = 0; i < 11; ++i) P.fix[i] = c->fix[i] ? 1 : 0;
+  for (int i = 0; i < 11; ++i) {
+    P.fix[i] = c->fix[i] ? 1 : 0;
+    P.fix_mask |= P.fix[i] << i;
+  }
   // FijaACeroDerivadasNoNecesarias (milosUtils.c:199-227)
   for (int k = 0; k < P.K; ++k) {
     if (P.K == 10 && k == 9) P.zero_row[k] = (P.fix[9] == 0 && P.fix[10] == 0);
     else P.zero_row[k] = (P.fix[k] == 0);
+    P.any_zero_row |= P.zero_row[k];
   }
   // me_der.c:499-525: the filling-factor row is 10 with NTERMS 11, else 9 unless
   // v_mac is inverted; row 9 is v_mac's with NTERMS 11 or 10 and alpha fixed
@@ -541,6 +545,7 @@ int run_streamed(pm_ctx* c, int64_t n, const float* spectro, const float* slight
   sio.jobs = static_cast<const PmJob*>(c->jobs.p);
   sio.jobs_cap = 1;
   sio.first_job = 0;
+  sio.max_pixels = int(std::min<int64_t>(n, INT32_MAX));
   sio.wait_limit_ns = 20000000000LL;
 
   // piece i holds first << i pixels (the last one the rest): at most `depth` pieces
@@ -805,6 +810,8 @@ int run_graph_small(pm_ctx* c, int64_t n, const float* spectro, const float* sli
       sio.q = q;
       sio.jobs = static_cast<const PmJob*>(c->jobs.p);
       sio.jobs_cap = 1;
+      sio.max_pixels = int(n);
+      sio.published = n;
       sio.wait_limit_ns = 20000000000LL;
       krc = pmk_invert_stream(*c->gs, sio, c->precision, c->tuning.variant, c->tuning.warps_per_block, false, s,
                               c->num_sms, nullptr);
@@ -951,6 +958,8 @@ int run_invert(pm_ctx* c, PmIO io, float* kernel_ms) {
   sio.jobs = static_cast<const PmJob*>(c->jobs.p);
   sio.jobs_cap = 1;
   sio.first_job = 0;
+  sio.max_pixels = int(std::min<int64_t>(io.npix, INT32_MAX));
+  sio.published = io.npix;
   sio.wait_limit_ns = 20000000000LL;
   PM_CUDA(cudaEventRecord(c->k0, c->stream), "event");
   if (c->P.classical) {
@@ -1260,7 +1269,7 @@ extern "C" int pm_autotune(pm_ctx* c, int64_t npix, const float* spectro, const 
   for (int variant : {0, 1, 2}) {
     if (!fp32 && variant != c->tuning.variant) continue;  // the FP64 kernel has one register budget
     for (int wpb : {1, 2, 4, 8, 16}) {
-      if ((variant == 2) != (wpb >= 8)) continue;  // lock-step blocks of 8 or 16 warps; 1, 2, 4 otherwise
+      if ((variant == 2) != (wpb >= 8)) continue;  // the block sizes of each variant
       for (int depth : {0, 2, 4}) {
         if (c->P.G != 1 && depth != 0) continue;  // multi-warp grids are not streamed
         cands.push_back(pm_tuning{variant, depth, wpb, c->tuning.graphs});

@@ -30,6 +30,8 @@ struct PmParams {
   int G;           // warps per pixel: 1 (nl <= 32), 2 (nl <= 64) or 4 (nl <= 128)
   int tap_lo, tap_hi;  // PSF support: taps outside [tap_lo, tap_hi] are below 1e-18 of the peak
   int fix[11];
+  int fix_mask;    // bit i: fix[i]
+  int any_zero_row;  // zero_row[] holds a nonzero entry
   int zero_row[PM_NTERMS_MAX];  // FijaACeroDerivadasNoNecesarias (milosUtils.c:199-227)
   int ff_row;      // RF row that holds d/d(filling factor), or -1
   int mac_row;     // 9 when RF row 9 is d/d(v_mac) (NTERMS 11, or 10 with alpha fixed), else -1
@@ -97,8 +99,9 @@ struct PmStreamIO {
   PmStreamQ* q;
   const PmJob* jobs;        // ring of jobs_cap descriptors; job k lives in slot k % jobs_cap
   int jobs_cap;
-  int pad_;
+  int max_pixels;           // no more pixels than this will be published (0: not known): no more warps are launched
   long long first_job;      // no ticket left belongs to a job before this one
+  long long published;      // every ticket, when all were published and the queue closed before the launch; else 0
   long long wait_limit_ns;  // longest wait for a ticket before giving up with PMQ_ERR_WAIT
 };
 

@@ -1,8 +1,8 @@
 // pm_stream.cu -- launches of the streamed inversion kernel (a persistent kernel
 // fed while it runs: pipelined host-buffer calls and the serving loop) for
-// normal Zeeman triplets, and the classical pre-pass.  Multiplets go to
-// pm_stream_zm.cu.
-#include "pm_stream_kernel.cuh"
+// normal Zeeman triplets (FP32: two pixels per warp; FP64: one), and the classical
+// pre-pass.  Multiplets go to pm_stream_zm.cu.
+#include "pm_pair_kernel.cuh"
 
 namespace {
 // Classical estimates (estimacionesClasicas + the NaN fixes of milos.c:975-983),
@@ -14,7 +14,8 @@ __global__ void __launch_bounds__(256) classical_prepass_kernel(const __grid_con
   const int lane = threadIdx.x & 31;
   const bool valid = lane < P.nl;
   const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-  for (long long pix = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); pix < npix; pix += nwarps) {
+  const int warp = __shfl_sync(kFull, int(threadIdx.x >> 5), 0);
+  for (long long pix = (long long)blockIdx.x * (blockDim.x >> 5) + warp; pix < npix; pix += nwarps) {
     const size_t base = size_t(pix) * 4 * P.nl;
     float O[4];
 #pragma unroll
@@ -38,49 +39,29 @@ __global__ void __launch_bounds__(256) classical_prepass_kernel(const __grid_con
 // MAC: the macroturbulence branch compiled in (a grid with a v_mac row).
 // pixgrid: per-pixel wavelengths (single-grid launches only).
 template <typename R, int KT, bool MAC>
-int launch_stream_any(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t st, int num_sms, int variant,
-                      int wpb, bool multi, size_t* smem_out, int reserve, bool pixgrid) {
-  if (pixgrid) {
-    if (multi) return snprintf(pmk_g_err, sizeof pmk_g_err, "pixel grids: single-grid launches only"), PM_EINVAL;
-    if constexpr (sizeof(R) == 4) {
-      return variant != 0  // 1, or 2 where no lock-step instance exists: the 128-register kernel
-                 ? launch_invert_stream<float, KT, 4, false, MAC, true>(GS, sio, st, num_sms, smem_out, wpb, reserve)
-                 : launch_invert_stream<float, KT, 3, false, MAC, true>(GS, sio, st, num_sms, smem_out, wpb, reserve);
-    } else {
-      return launch_invert_stream<double, KT, 1, false, MAC, true>(GS, sio, st, num_sms, smem_out, wpb, reserve);
-    }
-  }
+int launch_stream_any(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t st, int num_sms, int wpb, bool multi,
+                      size_t* smem_out, int reserve, bool pixgrid) {
+  if (pixgrid && multi) return snprintf(pmk_g_err, sizeof pmk_g_err, "pixel grids: single-grid launches only"), PM_EINVAL;
   if constexpr (sizeof(R) == 4) {
-    if constexpr (!MAC && KT <= 10) {
-      if (variant == 2) {  // lock-step blocks of wpb warps
-        if (multi) {
-          if (wpb == 16) return launch_invert_lockstep<float, KT, 16, true, MAC>(GS, sio, st, num_sms, smem_out, reserve);
-          if (wpb == 4) return launch_invert_lockstep<float, KT, 4, true, MAC>(GS, sio, st, num_sms, smem_out, reserve);
-          return launch_invert_lockstep<float, KT, 8, true, MAC>(GS, sio, st, num_sms, smem_out, reserve);
-        }
-        if (wpb == 16) return launch_invert_lockstep<float, KT, 16, false, MAC>(GS, sio, st, num_sms, smem_out, reserve);
-        if (wpb == 4) return launch_invert_lockstep<float, KT, 4, false, MAC>(GS, sio, st, num_sms, smem_out, reserve);
-        return launch_invert_lockstep<float, KT, 8, false, MAC>(GS, sio, st, num_sms, smem_out, reserve);
-      }
-    }
-    if (multi) return launch_invert_stream<float, KT, 4, true, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve);
-    return variant != 0 ? launch_invert_stream<float, KT, 4, false, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve)
-                        : launch_invert_stream<float, KT, 3, false, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve);
+    if (pixgrid) return launch_invert_pair<KT, false, MAC, true>(GS, sio, st, num_sms, smem_out, wpb, reserve);
+    return multi ? launch_invert_pair<KT, true, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve)
+                 : launch_invert_pair<KT, false, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve);
   } else {
+    if (pixgrid) return launch_invert_stream<double, KT, 1, false, MAC, true>(GS, sio, st, num_sms, smem_out, wpb, reserve);
     return multi ? launch_invert_stream<double, KT, 1, true, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve)
                  : launch_invert_stream<double, KT, 1, false, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve);
   }
 }
 
 template <typename R>
-int launch_stream_k(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t st, int num_sms, int variant, int wpb,
-                    bool multi, size_t* smem_out, int reserve, int K, bool mac, bool pg) {
+int launch_stream_k(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t st, int num_sms, int wpb, bool multi,
+                    size_t* smem_out, int reserve, int K, bool mac, bool pg) {
   // NTERMS 9 never has a v_mac row and 11 always has one (milos.c:152-157)
-  if (K == 9) return launch_stream_any<R, 9, false>(GS, sio, st, num_sms, variant, wpb, multi, smem_out, reserve, pg);
+  if (K == 9) return launch_stream_any<R, 9, false>(GS, sio, st, num_sms, wpb, multi, smem_out, reserve, pg);
   if (K == 10 && mac)
-    return launch_stream_any<R, 10, true>(GS, sio, st, num_sms, variant, wpb, multi, smem_out, reserve, pg);
-  if (K == 10) return launch_stream_any<R, 10, false>(GS, sio, st, num_sms, variant, wpb, multi, smem_out, reserve, pg);
-  if (K == 11) return launch_stream_any<R, 11, true>(GS, sio, st, num_sms, variant, wpb, multi, smem_out, reserve, pg);
+    return launch_stream_any<R, 10, true>(GS, sio, st, num_sms, wpb, multi, smem_out, reserve, pg);
+  if (K == 10) return launch_stream_any<R, 10, false>(GS, sio, st, num_sms, wpb, multi, smem_out, reserve, pg);
+  if (K == 11) return launch_stream_any<R, 11, true>(GS, sio, st, num_sms, wpb, multi, smem_out, reserve, pg);
   snprintf(pmk_g_err, sizeof pmk_g_err, "nterms=%d has no compiled kernel", K);
   return PM_ENOTSUP;
 }
@@ -116,8 +97,8 @@ int pmk_invert_stream(const PmGridSet& GS, const PmStreamIO& sio, int precision,
     return pmk_invert_stream_zm(GS, sio, precision, wpb, multi, stream, num_sms, smem_out, reserve_blocks, pixgrid,
                                 mac);
   if (precision == PM_PREC_FP32)
-    return launch_stream_k<float>(GS, sio, st, num_sms, variant, wpb, multi, smem_out, reserve_blocks, K, mac, pixgrid);
-  return launch_stream_k<double>(GS, sio, st, num_sms, variant, wpb, multi, smem_out, reserve_blocks, K, mac, pixgrid);
+    return launch_stream_k<float>(GS, sio, st, num_sms, wpb, multi, smem_out, reserve_blocks, K, mac, pixgrid);
+  return launch_stream_k<double>(GS, sio, st, num_sms, wpb, multi, smem_out, reserve_blocks, K, mac, pixgrid);
 }
 
 
