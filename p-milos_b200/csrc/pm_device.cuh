@@ -331,17 +331,38 @@ struct alignas(16) BlockSmem {
 // State of the damped solve: the normal equations and the Jacobi rotation tables.
 struct alignas(16) SolveSmem {
   double ab[PM_NTERMS_MAX * PM_NTERMS_MAX + PM_NTERMS_MAX];  // alpha (K*K) then beta (K)
-  double rot[12][3];      // per index: partner, c, signed s
-  int pq[6][2];           // the rotated pairs of the current round
+  double2 rot[12];        // per index: c, signed s of the current round
+  double diag[12];        // the rotated diagonal
+  int2 pq[6];             // the rotated pairs
+  int mate[12];           // per index: the other one of its pair
   double delta[PM_NTERMS_MAX];
 };
 
+// tr: response functions [profile][lambda] (transpose buffer; scratch of the
+// solvers and of the normal equations); ls: the synthesis state that the response
+// functions are formed from, per lane.  They share their memory (every lane has its
+// state in registers when the first profile is stored), except (APART) in kernels
+// with a macroturbulence branch, which uses tr before, and in those of multiplets,
+// whose roundings one more barrier there would change.
+template <typename R, bool APART>
+struct WarpRows {
+  static constexpr bool kSharedRows = false;
+  R tr[NL * TRS];
+  R ls[NL][kLaneStatePad];
+};
 template <typename R>
-struct alignas(16) WarpSmem {
-  R tr[NL * TRS];       // response functions: [profile][lambda] (transpose buffer)
-  R xs[4][XSR];         // padded Stokes rows for the synthesis PSF correlation
+struct WarpRows<R, false> {
+  static constexpr bool kSharedRows = true;
+  union {
+    R tr[NL * TRS];
+    R ls[NL][kLaneStatePad];
+  };
+};
+
+template <typename R, bool APART>
+struct alignas(16) WarpSmem : WarpRows<R, APART> {
   SolveSmem sv;
-  R ls[NL][kLaneStatePad];    // synthesis state the response functions need, per lane
+  R xs[4][XSR];         // padded Stokes rows for the synthesis PSF correlation
   ModelTerms<R> mt;           // per-model terms of the last synthesis (uniform)
   double model[11], trial[11];
   // the streamed kernel's place in the ticket stream: kept here rather than in
@@ -358,10 +379,10 @@ struct alignas(16) WarpSmem {
 // region, every xs row and every rv row to start on a 16-byte boundary.
 template <typename R>
 constexpr bool smem_layout_ok() {
-  return sizeof(BlockSmem<R>) % 16 == 0 && sizeof(WarpSmem<R>) % 16 == 0 &&
-         offsetof(WarpSmem<R>, xs) % 16 == 0 && (XSR * sizeof(R)) % 16 == 0 &&
-         offsetof(WarpSmem<R>, ls) % 16 == 0 && offsetof(WarpSmem<R>, mt) % 16 == 0 &&
-         ((64 + BlockSmem<R>::VEC) * sizeof(R)) % 16 == 0;
+  return sizeof(BlockSmem<R>) % 16 == 0 && sizeof(WarpSmem<R, false>) % 16 == 0 && sizeof(WarpSmem<R, true>) % 16 == 0 &&
+         sizeof(WarpRows<R, false>) % 16 == 0 && sizeof(WarpRows<R, true>) % 16 == 0 &&
+         (NL * TRS * sizeof(R)) % 16 == 0 && sizeof(SolveSmem) % 16 == 0 && (XSR * sizeof(R)) % 16 == 0 &&
+         sizeof(LaneState<R>) % 16 == 0 && ((64 + BlockSmem<R>::VEC) * sizeof(R)) % 16 == 0;
 }
 static_assert(smem_layout_ok<float>(), "shared-memory layout breaks 16-byte vector loads (float)");
 static_assert(smem_layout_ok<double>(), "shared-memory layout breaks 16-byte vector loads (double)");
@@ -395,8 +416,8 @@ __device__ __forceinline__ const float* slight_of(const PmParams& P, const Block
 // Lane l computes outputs 4c..4c+3 (c = l & 7) of Stokes l >> 3 from one aligned
 // 36-sample window: 9 vector loads and 128 FMAs whose taps are compile-time
 // indexed constant operands.
-template <typename R>
-__device__ __forceinline__ void psf_rows(const PmParams& P, WarpSmem<R>& sm, int lane, bool valid, R S[4]) {
+template <typename R, typename SM>
+__device__ __forceinline__ void psf_rows(const PmParams& P, SM& sm, int lane, bool valid, R S[4]) {
   const R i0 = __shfl_sync(kFull, S[0], 0), in = __shfl_sync(kFull, S[0], P.nl - 1);
   const R ic = (i0 > in) ? i0 : in;
   const int off = NL + (P.half & 3);  // data at xs[s][off + i]; off - half is a multiple of 4
@@ -424,12 +445,16 @@ __device__ __forceinline__ void psf_rows(const PmParams& P, WarpSmem<R>& sm, int
 #pragma unroll
     for (int kk = 0; kk < 4; ++kk) acc[kk] = fma(g, w[kk + j], acc[kk]);
   }
-  R* o = sm.tr;  // scratch [4][NL]
+  // the outputs through tr, or (where tr holds the synthesis states) back into the
+  // rows, once every window is read
+  R* o = SM::kSharedRows ? &sm.xs[0][off] : sm.tr;
+  constexpr int os = SM::kSharedRows ? XSR : NL;
+  if constexpr (SM::kSharedRows) __syncwarp();
 #pragma unroll
-  for (int kk = 0; kk < 4; ++kk) o[st * NL + 4 * c + kk] = (st == 0) ? ic - acc[kk] : acc[kk];
+  for (int kk = 0; kk < 4; ++kk) o[st * os + 4 * c + kk] = (st == 0) ? ic - acc[kk] : acc[kk];
   __syncwarp();
 #pragma unroll
-  for (int s = 0; s < 4; ++s) S[s] = valid ? o[s * NL + lane] : R(0);
+  for (int s = 0; s < 4; ++s) S[s] = valid ? o[s * os + lane] : R(0);
   __syncwarp();
 }
 
@@ -601,8 +626,8 @@ __device__ __forceinline__ void synthesize_terms(const PmParams& P, SM& sm, cons
   __syncwarp();
 }
 
-template <typename R, bool MAC = false, bool ZM = false>
-__device__ __forceinline__ void synthesize(const PmParams& P, WarpSmem<R>& sm, const double* m,
+template <typename R, bool MAC, bool ZM, typename SM>
+__device__ __forceinline__ void synthesize(const PmParams& P, SM& sm, const double* m,
                                            const float* sl_pix, int lane, bool valid, double dl, R S[4], R Su[4]) {
   ModelTerms<R> T;
   model_terms<R, ZM>(P, m, T);
@@ -614,8 +639,8 @@ __device__ __forceinline__ void synthesize(const PmParams& P, WarpSmem<R>& sm, c
   }, [&] { psf_rows<R>(P, sm, lane, valid, S); });
 }
 
-template <typename R>
-__device__ __forceinline__ void load_lane_state(const WarpSmem<R>& sm, int lane, LaneState<R>& st) {
+template <typename R, typename SM>
+__device__ __forceinline__ void load_lane_state(const SM& sm, int lane, LaneState<R>& st) {
   copy16(st, *reinterpret_cast<const LaneState<R>*>(sm.ls[lane]));
 }
 
@@ -729,9 +754,8 @@ __device__ __forceinline__ void rf_lane(const PmParams& P, const ModelTerms<R>& 
 // adds its products in the order of m, so the results are those of the one-input
 // loop bit for bit.  Stokes-I rows correlate Ic - x with Ic = max of the row's end
 // points.
-template <typename R>
-__device__ __forceinline__ void rf_correlate(const PmParams& P, const BlockSmem<R>& bs, WarpSmem<R>& sm,
-                                             int lane) {
+template <typename R, typename SM>
+__device__ __forceinline__ void rf_correlate(const PmParams& P, const BlockSmem<R>& bs, SM& sm, int lane) {
   constexpr int VEC = BlockSmem<R>::VEC;
   __syncwarp();
   R* row = sm.tr + lane * TRS;
@@ -849,8 +873,8 @@ __device__ __forceinline__ void transpose_reduce(T (&v)[N], int lane) {
 
 // Response functions at this lane's wavelength after correlation, filling factor
 // and FijaACeroDerivadasNoNecesarias: d[row][stokes] for rows 0..K-1.
-template <typename R, int KT>
-__device__ __forceinline__ void gather_rf(const PmParams& P, const WarpSmem<R>& sm, int lane, bool valid,
+template <typename R, int KT, typename SM>
+__device__ __forceinline__ void gather_rf(const PmParams& P, const SM& sm, int lane, bool valid,
                                           R alf, const R Sff[4], const float* sl_pix, const R (&dmac)[4],
                                           R (&d)[KT][4]) {
   const R* col = sm.tr + lane;
@@ -936,8 +960,8 @@ __device__ __forceinline__ void ne_reduce_chunk(double* red, int lane, const R (
 // Normal equations (covarm2): alpha = sum w_s/sigma^2 d_a d_b (upper triangle),
 // beta = sum w_s (S - O)/sigma^2 d_b, reduced over the warp in chunks of 32
 // entries (31 shuffles each) and stored in FP64.
-template <typename R, int KT>
-__device__ __forceinline__ void normal_eq(const PmParams& P, WarpSmem<R>& sm, int lane, const R (&d)[KT][4],
+template <typename R, int KT, typename SM>
+__device__ __forceinline__ void normal_eq(const PmParams& P, SM& sm, int lane, const R (&d)[KT][4],
                                           const R S[4], const float O[4], const R isig[4]) {
   constexpr int NA = KT * (KT + 1) / 2;
   constexpr int NT = NA + KT;
@@ -990,7 +1014,11 @@ __device__ __forceinline__ double chisq(const PmParams& P, const R S[4], const f
 // Symmetric eigen-decomposition by parallel-ordered Jacobi (round-robin pairs,
 // all K/2 rotations of a round applied at once), then the pseudo-inverse with
 // the absolute 1e-12 eigenvalue cut of mil_svd.  Warp-cooperative; every lane
-// returns delta.
+// returns delta.  Bound by a round's serial chain (two divisions, a square root and
+// a reciprocal one for the angle, then the update), 9 rounds a sweep: a lane keeps
+// its entries' indices, the two copies of A change places instead of being copied
+// back, and a round has two barriers (500 pixels with this solve in every step,
+// 14,906 steps: 4.85 -> 2.65 ms).
 template <int KT>
 constexpr int eigen_scratch_doubles() {
   return 3 * ((KT + 1) & ~1) * ((KT + 1) & ~1);
@@ -999,80 +1027,116 @@ constexpr int eigen_scratch_doubles() {
 template <int KT>
 __device__ __noinline__ void solve_eigen(SolveSmem& sm, double* scratch, int lane, double flambda) {
   constexpr int M = (KT + 1) & ~1;  // padded to even; index KT (if any) is a dummy
+  constexpr int NE = (M * M + 31) / 32, NV = (M * (M / 2) + 31) / 32;  // entries of A, items of V per lane
   double* A = scratch;  // eigen_scratch_doubles<KT>() doubles, idle otherwise during the solve
   double* V = A + M * M;
   double* A2 = V + M * M;
-  for (int e = lane; e < M * M; e += 32) {
-    const int i = e / M, j = e % M;
-    double a = 0;
-    if (i < KT && j < KT) {
-      a = sm.ab[i * KT + j];
-      if (i == j) a *= (1.0 + flambda);
+  // this lane's entries of A (row, column) and items of V (row, pair), fixed
+  int ei[NE], ej[NE], vi[NV], vk[NV];
+#pragma unroll
+  for (int q = 0; q < NE; ++q) {
+    const int e = lane + 32 * q;
+    ei[q] = e / M;
+    ej[q] = e % M;
+    if (e < M * M) {
+      double a = 0;
+      if (ei[q] < KT && ej[q] < KT) {
+        a = sm.ab[ei[q] * KT + ej[q]];
+        if (ei[q] == ej[q]) a *= (1.0 + flambda);
+      }
+      A[e] = a;
+      V[e] = (ei[q] == ej[q]) ? 1.0 : 0.0;
     }
-    A[e] = a;
-    V[e] = (i == j) ? 1.0 : 0.0;
   }
+#pragma unroll
+  for (int q = 0; q < NV; ++q) {
+    const int e = lane + 32 * q;
+    vi[q] = e / (M / 2);
+    vk[q] = e % (M / 2);
+  }
+  // the circle method: position 0 fixed, positions 1..M-1 rotate; M - 1 rounds come
+  // round to the first pairing
+  int pa = lane, pb = M - 1 - lane;
   __syncwarp();
   for (int sweep = 0; sweep < 24; ++sweep) {
     double off = 0, dg = 0;
-    for (int e = lane; e < KT * KT; e += 32) {
-      const int i = e / KT, j = e % KT;
-      const double a = A[i * M + j];
-      if (i == j) dg += a * a;
-      else if (i < j) off += a * a;
+#pragma unroll
+    for (int q = 0; q < (KT * KT + 31) / 32; ++q) {
+      const int e = lane + 32 * q;
+      if (e < KT * KT) {
+        const int i = e / KT, j = e % KT;
+        const double a = A[i * M + j];
+        if (i == j) dg = fma(a, a, dg);
+        else if (i < j) off = fma(a, a, off);
+      }
     }
     off = warp_sum(off);
     dg = warp_sum(dg);
-    if (off == 0.0 || off <= 1e-36 * dg) break;
+    if (uniform(off == 0.0 || off <= 1e-36 * dg)) break;
+#pragma unroll 1
     for (int r = 0; r < M - 1; ++r) {
-      // circle method: position 0 fixed, positions 1..M-1 rotate
       if (lane < M / 2) {
-        const int k = lane;
-        const int pa = (k == 0) ? 0 : ((k - 1 + r) % (M - 1)) + 1;
-        const int pb = ((M - 1 - k - 1 + r) % (M - 1)) + 1;
         const int p = pa < pb ? pa : pb, q = pa < pb ? pb : pa;
         double c = 1.0, s = 0.0, t = 0.0;
         const double apq = (p < KT && q < KT) ? A[p * M + q] : 0.0;
+        const double app = A[p * M + p], aqq = A[q * M + q];
         if (apq != 0.0) {
-          const double app = A[p * M + p], aqq = A[q * M + q];
           const double theta = (aqq - app) / (2.0 * apq);
-          t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(theta * theta + 1.0));
+          t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(fma(theta, theta, 1.0)));
           if (!isfinite(t)) t = 0.0;
-          c = rsqrt(t * t + 1.0);
+          c = rsqrt(fma(t, t, 1.0));
           s = t * c;
         }
         // column p of J: (c at p, -s at q); column q: (s at p, c at q)
-        sm.rot[p][0] = q; sm.rot[p][1] = c; sm.rot[p][2] = -s;
-        sm.rot[q][0] = p; sm.rot[q][1] = c; sm.rot[q][2] = s;
-        sm.pq[k][0] = p; sm.pq[k][1] = q;
-        // exact diagonal update (Rutishauser) stored in the unused slot of delta
-        if (p < KT) sm.delta[p] = A[p * M + p] - t * apq;
-        if (q < KT) sm.delta[q] = A[q * M + q] + t * apq;
+        sm.rot[p] = make_double2(c, -s);
+        sm.rot[q] = make_double2(c, s);
+        sm.mate[p] = q;
+        sm.mate[q] = p;
+        sm.pq[lane] = make_int2(p, q);
+        // exact diagonal update (Rutishauser): with a dummy index (whose entry stays
+        // zero) one product per entry, fused, else one rounded product for both
+        if constexpr (M != KT) {
+          sm.diag[p] = p < KT ? fma(-t, apq, app) : 0.0;
+          sm.diag[q] = q < KT ? fma(t, apq, aqq) : 0.0;
+        } else {
+          const double tp = __dmul_rn(t, apq);
+          sm.diag[p] = app - tp;
+          sm.diag[q] = aqq + tp;
+        }
+        if (lane) pa = pa == M - 1 ? 1 : pa + 1;
+        pb = pb == M - 1 ? 1 : pb + 1;
       }
       __syncwarp();
-      for (int e = lane; e < M * M; e += 32) {
-        const int i = e / M, j = e % M;
-        const int pi = int(sm.rot[i][0]), pj = int(sm.rot[j][0]);
-        const double ci = sm.rot[i][1], si = sm.rot[i][2], cj = sm.rot[j][1], sj = sm.rot[j][2];
-        double a;
-        if (i == j) a = (i < KT) ? sm.delta[i] : 0.0;
-        else if (pi == j) a = 0.0;
-        else
-          a = ci * (cj * A[i * M + j] + sj * A[i * M + pj]) + si * (cj * A[pi * M + j] + sj * A[pi * M + pj]);
-        A2[e] = a;
+      // A2 <- J^T A J
+#pragma unroll
+      for (int q = 0; q < NE; ++q) {
+        const int i = ei[q], j = ej[q];
+        if (NE * 32 == M * M || q + 1 < NE || i < M) {
+          const int pi = sm.mate[i], pj = sm.mate[j];
+          const double2 ri = sm.rot[i], rj = sm.rot[j];
+          const double x = fma(rj.x, A[i * M + j], __dmul_rn(rj.y, A[i * M + pj]));
+          const double y = fma(rj.x, A[pi * M + j], __dmul_rn(rj.y, A[pi * M + pj]));
+          const double a = fma(ri.x, x, __dmul_rn(ri.y, y));
+          A2[i * M + j] = i == j ? sm.diag[i] : pi == j ? 0.0 : a;
+        }
       }
       // V <- V J, one work item per (row, rotated pair): both columns of the pair
       // are rewritten from their old values by the same lane
-      for (int e = lane; e < M * (M / 2); e += 32) {
-        const int i = e / (M / 2), k = e % (M / 2);
-        const int p = sm.pq[k][0], q = sm.pq[k][1];
-        const double vp = V[i * M + p], vq = V[i * M + q];
-        V[i * M + p] = vp * sm.rot[p][1] + vq * sm.rot[p][2];
-        V[i * M + q] = vq * sm.rot[q][1] + vp * sm.rot[q][2];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        if (q + 1 < NV || vi[q] < M) {
+          const int2 k = sm.pq[vk[q]];
+          double* row = V + vi[q] * M;
+          const double vp = row[k.x], vq = row[k.y];
+          const double2 rp = sm.rot[k.x], rq = sm.rot[k.y];
+          row[k.x] = fma(vp, rp.x, __dmul_rn(vq, rp.y));
+          row[k.y] = fma(vq, rq.x, __dmul_rn(vp, rq.y));
+        }
       }
       __syncwarp();
-      for (int e = lane; e < M * M; e += 32) A[e] = A2[e];
-      __syncwarp();
+      double* other = A;
+      A = A2;
+      A2 = other;
     }
   }
   // pseudo-inverse: aux_j = (V^T beta)_j / w_j (0 if |w_j| <= 1e-12); delta = V aux
@@ -1081,12 +1145,12 @@ __device__ __noinline__ void solve_eigen(SolveSmem& sm, double* scratch, int lan
     double sum = 0;
     for (int i = 0; i < KT; ++i) sum += beta[i] * V[i * M + lane];
     const double w = A[lane * M + lane];
-    sm.rot[lane][0] = sum * ((fabs(w) > 1e-12) ? (1.0 / w) : 0.0);
+    sm.diag[lane] = sum * ((fabs(w) > 1e-12) ? (1.0 / w) : 0.0);
   }
   __syncwarp();
   if (lane < KT) {
     double sum = 0;
-    for (int j = 0; j < KT; ++j) sum += V[lane * M + j] * sm.rot[j][0];
+    for (int j = 0; j < KT; ++j) sum += V[lane * M + j] * sm.diag[j];
     sm.delta[lane] = sum;
   }
   __syncwarp();
@@ -1315,8 +1379,8 @@ __device__ __forceinline__ void classical(const PmParams& P, const float O[4], i
 // macroturbulence convolutions, the v_mac row and the filling-factor terms.
 // m must be the model of the last synthesis.  MAC: compiled with the
 // macroturbulence branch (the grid has a v_mac row; NTERMS >= 10).
-template <typename R, int KT, bool MAC = (KT >= 10), bool ZM = false>
-__device__ __forceinline__ void response_rows(const PmParams& P, const BlockSmem<R>& bs, WarpSmem<R>& sm, int lane,
+template <typename R, int KT, bool MAC, bool ZM, typename SM>
+__device__ __forceinline__ void response_rows(const PmParams& P, const BlockSmem<R>& bs, SM& sm, int lane,
                                               bool valid, const double* m, double dl, const R Sff[4],
                                               const float* sl_pix, R (&d)[KT][4]) {
   const bool mac_on = MAC && m[9] > kMacMin;
@@ -1327,6 +1391,7 @@ __device__ __forceinline__ void response_rows(const PmParams& P, const BlockSmem
     copy16(T, sm.mt);
     LaneState<R> st;
     load_lane_state<R>(sm, lane, st);
+    if constexpr (SM::kSharedRows) __syncwarp();
     rf_lane<R, TRS, ZM>(P, T, st, sm.tr + lane, valid);
     alf = T.alf;
   }
@@ -1343,8 +1408,8 @@ __device__ __forceinline__ void response_rows(const PmParams& P, const BlockSmem
 }
 
 // Response functions at the current synthesis -> alpha, beta in shared memory.
-template <typename R, int KT, bool MAC, bool ZM>
-__device__ __forceinline__ void rf_and_normal_eq(const PmParams& P, const BlockSmem<R>& bs, WarpSmem<R>& sm,
+template <typename R, int KT, bool MAC, bool ZM, typename SM>
+__device__ __forceinline__ void rf_and_normal_eq(const PmParams& P, const BlockSmem<R>& bs, SM& sm,
                                                  int lane, bool valid, double dl, const R S[4], const R Sff[4],
                                                  const float O[4], const R isig[4], const float* sl_pix) {
   R d[KT][4];
@@ -1356,11 +1421,6 @@ __device__ __forceinline__ void rf_and_normal_eq(const PmParams& P, const BlockS
       for (int s = 0; s < 4; ++s) d[r][s] = 0;
     }
   normal_eq<R, KT>(P, sm, lane, d, S, O, isig);
-}
-
-template <typename R>
-__device__ __forceinline__ WarpSmem<R>& warp_smem(unsigned char* raw, int warp) {
-  return reinterpret_cast<WarpSmem<R>*>(raw + sizeof(BlockSmem<R>))[warp];
 }
 
 // A pointer field of a job descriptor, read from L2 (the host may have written
@@ -1383,8 +1443,8 @@ __device__ __forceinline__ T* ld_ptr(T* const* p) {
 // kept in a register; otherwise the grid's offsets are read from the
 // parameter block where they are used.
 // ZM: the line is a Zeeman multiplet.
-template <typename R, int KT, bool MAC, bool PIXGRID, bool ZM = false>
-__device__ __forceinline__ void invert_pixel(const PmParams& P, const BlockSmem<R>& bs, WarpSmem<R>& sm, int lane,
+template <typename R, int KT, bool MAC, bool PIXGRID, bool ZM, typename SM>
+__device__ __forceinline__ void invert_pixel(const PmParams& P, const BlockSmem<R>& bs, SM& sm, int lane,
                                              unsigned long long* ctr) {
   const bool valid = lane < P.nl;
   double* m = sm.model;

@@ -12,7 +12,8 @@ __global__ void __launch_bounds__(128) synth_kernel(const __grid_constant__ PmPa
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   BlockSmem<R>& bs = *reinterpret_cast<BlockSmem<R>*>(smem_raw);
-  WarpSmem<R>& sm = warp_smem<R>(smem_raw, warp);
+  using SM = WarpSmem<R, (KT >= 10 || ZM)>;
+  SM& sm = reinterpret_cast<SM*>(smem_raw + sizeof(BlockSmem<R>))[warp];
   load_taps<R>(P, bs);
   for (int e = lane; e < 4 * XSR; e += 32) (&sm.xs[0][0])[e] = R(0);
   if (lane == 0) sm.xs_dirty = 0;
@@ -51,7 +52,7 @@ __global__ void __launch_bounds__(128) synth_kernel(const __grid_constant__ PmPa
 template <typename R, int KT, bool ZM>
 int launch_synth(const PmParams& P, const PmIO& io, cudaStream_t st) {
   const int threads = 128;
-  const size_t smem = sizeof(BlockSmem<R>) + sizeof(WarpSmem<R>) * (threads / 32);
+  const size_t smem = sizeof(BlockSmem<R>) + sizeof(WarpSmem<R, (KT >= 10 || ZM)>) * (threads / 32);
   auto kern = synth_kernel<R, KT, ZM>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
   if (e != cudaSuccess) return snprintf(pmk_g_err, sizeof pmk_g_err, "%s", cudaGetErrorString(e)), PM_EIO;

@@ -65,8 +65,8 @@ struct GridParams {
 
 // The warp's pixel is finished: count it on its job and, when it was the job's
 // last pixel, raise the job's host flag (the server's completion signal).
-template <typename R>
-__device__ __forceinline__ void job_pixel_done(WarpSmem<R>& sm, int lane) {
+template <typename SM>
+__device__ __forceinline__ void job_pixel_done(SM& sm, int lane) {
   const PmJob* jp = *reinterpret_cast<const PmJob* const volatile*>(&sm.job);
   unsigned long long* done = ld_ptr(&jp->done);
   if (done) {
@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(128, MINB) invert_stream_kernel(
   constexpr int NG = MULTI ? PMK_MAX_GRIDS : 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   BlockSmem<R>* bs = reinterpret_cast<BlockSmem<R>*>(smem_raw);
-  WarpSmem<R>& sm = reinterpret_cast<WarpSmem<R>*>(smem_raw + NG * sizeof(BlockSmem<R>))[warp];
+  using SM = WarpSmem<R, MAC || ZM>;
+  SM& sm = reinterpret_cast<SM*>(smem_raw + NG * sizeof(BlockSmem<R>))[warp];
 #pragma unroll 1
   for (int g = 0; g < NG && g < GS.ngrids; ++g) load_taps<R>(GS.g[g], bs[g]);
   __syncthreads();
@@ -151,7 +152,7 @@ int launch_invert_stream(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_
                          size_t* smem_out, int wpb, int reserve) {
   if (wpb > 4) wpb = 4;  // at most 4 warps per block
   const int threads = 32 * wpb;
-  const size_t smem = (MULTI ? PMK_MAX_GRIDS : 1) * sizeof(BlockSmem<R>) + sizeof(WarpSmem<R>) * (threads / 32);
+  const size_t smem = (MULTI ? PMK_MAX_GRIDS : 1) * sizeof(BlockSmem<R>) + sizeof(WarpSmem<R, MAC || ZM>) * (threads / 32);
   if (smem_out) *smem_out = smem;
   auto kern = invert_stream_kernel<R, KT, MINB, MULTI, MAC, PIXGRID, ZM>;
   constexpr int NG = MULTI ? PMK_MAX_GRIDS : 1;
