@@ -47,9 +47,14 @@ int launch_stream_any(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t s
     return multi ? launch_invert_pair<KT, true, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve)
                  : launch_invert_pair<KT, false, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve);
   } else {
-    if (pixgrid) return launch_invert_stream<double, KT, 1, false, MAC, true>(GS, sio, st, num_sms, smem_out, wpb, reserve);
-    return multi ? launch_invert_stream<double, KT, 1, true, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve)
-                 : launch_invert_stream<double, KT, 1, false, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve);
+    // three blocks per SM (168 registers, spills around the normal equations): the
+    // serial solve gains more by 12 warps than the rest loses (4,096 pixels, eigen
+    // solve: 6.48 ms with two blocks, 5.50 with three; Cholesky, 3,000 pixels: 2.00,
+    // 1.90).  With a macroturbulence branch shared memory allows two blocks only.
+    constexpr int MINB = MAC ? 1 : 3;
+    if (pixgrid) return launch_invert_stream<double, KT, MINB, false, MAC, true>(GS, sio, st, num_sms, smem_out, wpb, reserve);
+    return multi ? launch_invert_stream<double, KT, MINB, true, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve)
+                 : launch_invert_stream<double, KT, MINB, false, MAC>(GS, sio, st, num_sms, smem_out, wpb, reserve);
   }
 }
 
