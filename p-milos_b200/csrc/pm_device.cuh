@@ -54,6 +54,9 @@ constexpr double kGhostSigma = 1e21;
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kLaneStateWords = 35;  // words of LaneState (synthesis state kept for the RFs)
 constexpr int kLaneStatePad = 36;    // row stride: 16-byte rows, conflict-free 128-bit access
+// Row stride of a 32-column float buffer whose vector reads along a row and accesses
+// down a column are both conflict-free.
+constexpr int kRow = NL + 4;
 
 // Hui, Armstrong & Wray (1978) rational approximation of w(z), z = a - i v:
 // numerator degree 6, monic denominator degree 7 (published coefficients).
@@ -946,6 +949,24 @@ template <typename R, int KT, int CH, int... I>
 __device__ __forceinline__ void ne_chunk(R (&v)[32], const R (&d)[KT][4], const R (&cw)[4], const R (&rw)[4],
                                          std::integer_sequence<int, I...>) {
   ((v[I] = ne_entry<R, KT, CH * 32 + I>(d, cw, rw)), ...);
+}
+
+// The sum over the warp of entry `lane` of the 32 rows in buf: the tree of a
+// butterfly over lanes (distances 16, 8, 4, 2, 1), in packed additions.
+__device__ __forceinline__ float ne_row_sum(const float* buf, int lane) {
+  const float4* r = reinterpret_cast<const float4*>(buf + lane * kRow);
+  float2 a[8];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float4 lo = r[i], hi = r[i + 4];
+    a[2 * i] = __fadd2_rn(make_float2(lo.x, lo.y), make_float2(hi.x, hi.y));
+    a[2 * i + 1] = __fadd2_rn(make_float2(lo.z, lo.w), make_float2(hi.z, hi.w));
+  }
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1)
+#pragma unroll
+    for (int i = 0; i < h; ++i) a[i] = __fadd2_rn(a[i], a[i + h]);
+  return a[0].x + a[0].y;
 }
 
 template <typename R, int KT, int CH>

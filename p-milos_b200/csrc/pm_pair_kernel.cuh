@@ -15,8 +15,6 @@
 
 namespace {
 
-// Row stride of tr: 16-byte rows whose vector reads and column reads are conflict-free.
-constexpr int kRow = NL + 4;
 static_assert(kRow == kLaneStatePad, "the response functions overwrite the synthesis states row by row");
 
 // Per block: the PSF taps, centred and reversed, so that the window of a group of
@@ -403,24 +401,6 @@ __device__ __forceinline__ void ne_add(float (&acc)[KT * (KT + 1) / 2 + KT], con
       ne_add<KT, E + 1>(acc, d, c, r);
     }
   }
-}
-
-// The sum over the warp of entry `lane` of the 32 rows in buf: the tree of a
-// butterfly over lanes (distances 16, 8, 4, 2, 1), in packed additions.
-__device__ __forceinline__ float ne_row_sum(const float* buf, int lane) {
-  const float4* r = reinterpret_cast<const float4*>(buf + lane * kRow);
-  float2 a[8];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float4 lo = r[i], hi = r[i + 4];
-    a[2 * i] = __fadd2_rn(make_float2(lo.x, lo.y), make_float2(hi.x, hi.y));
-    a[2 * i + 1] = __fadd2_rn(make_float2(lo.z, lo.w), make_float2(hi.z, hi.w));
-  }
-#pragma unroll
-  for (int h = 4; h > 0; h >>= 1)
-#pragma unroll
-    for (int i = 0; i < h; ++i) a[i] = __fadd2_rn(a[i], a[i + h]);
-  return a[0].x + a[0].y;
 }
 
 // Normal equations (covarm2): alpha = sum w_s/sigma^2 d_a d_b (upper triangle), beta

@@ -397,9 +397,64 @@ __device__ __forceinline__ void rf_wide(const PmParams& P, WideSmem<R, G>& sm, i
   }
 }
 
-// Normal equations over the block: packed entries reduced per warp (as
-// normal_eq), then the G warp totals summed in warp order into sv.ab.
-template <typename R, int KT, int G>
+// Entries E and E + 1 (columns b and b + 1 of one row) of the packed normal
+// equations with packed f32x2 products; each half rounds as ne_entry's.
+template <int KT, int E>
+__device__ __forceinline__ float2 ne_entry2(const float (&d)[KT][4], const float (&cw)[4], const float (&rw)[4]) {
+  constexpr int a = ne_row(E, KT), b = ne_col(E, KT);
+  float2 acc = make_float2(0.0f, 0.0f);
+#pragma unroll
+  for (int s = 0; s < 4; ++s) {
+    const float2 db = make_float2(d[b][s], d[b + 1][s]);
+    if constexpr (a < KT)
+      acc = __ffma2_rn(__fmul2_rn(make_float2(d[a][s], d[a][s]), db), make_float2(cw[s], cw[s]), acc);
+    else
+      acc = __ffma2_rn(make_float2(rw[s], rw[s]), db, acc);
+  }
+  return acc;
+}
+
+// Entries I.. of chunk CH at this lane's wavelength into column `lane` of buf.
+template <int KT, int CH, int I>
+__device__ __forceinline__ void ne_store(float* buf, int lane, const float (&d)[KT][4], const float (&cw)[4],
+                                         const float (&rw)[4]) {
+  constexpr int E = CH * 32 + I, NE = KT * (KT + 1) / 2 + KT;
+  if constexpr (I < 32 && E < NE) {
+    constexpr int b = ne_col(E, KT);
+    if constexpr (b % 2 == 0 && b + 1 < KT && I + 1 < 32) {
+      const float2 v = ne_entry2<KT, E>(d, cw, rw);
+      buf[I * kRow + lane] = v.x;
+      buf[(I + 1) * kRow + lane] = v.y;
+      ne_store<KT, CH, I + 2>(buf, lane, d, cw, rw);
+    } else {
+      buf[I * kRow + lane] = ne_entry<float, KT, E>(d, cw, rw);
+      ne_store<KT, CH, I + 1>(buf, lane, d, cw, rw);
+    }
+  }
+}
+
+// The warp's sums of the packed entries into mine, 32 at a time transposed through
+// buf (32 rows of kRow floats of this warp's own): 56 instructions per 32 entries,
+// where ne_reduce_chunk's shuffles take 124; the order of the additions is its.
+template <int KT, int CH>
+__device__ __forceinline__ void ne_warp_sums(int lane, const float (&d)[KT][4], const float (&cw)[4],
+                                             const float (&rw)[4], float* buf, double* mine) {
+  constexpr int NE = KT * (KT + 1) / 2 + KT;
+  if constexpr (CH * 32 < NE) {
+    __syncwarp();  // buf is read no more
+    ne_store<KT, CH, 0>(buf, lane, d, cw, rw);
+    __syncwarp();
+    const float v = ne_row_sum(buf, lane);
+    if (CH * 32 + lane < NE) mine[CH * 32 + lane] = double(v);
+    ne_warp_sums<KT, CH + 1>(lane, d, cw, rw, buf, mine);
+  }
+}
+
+// Normal equations over the block: packed entries reduced per warp (in FP32 through
+// the warp's synthesis states, which the response functions have read; in FP64 and
+// with a v_mac row as normal_eq), then the G warp totals summed in warp order into
+// sv.ab.
+template <typename R, int KT, int G, bool MAC>
 __device__ __forceinline__ void normal_eq_wide(const PmParams& P, WideSmem<R, G>& sm, int& slot,
                                                const R (&d)[KT][4], const R S[4], const float O[4],
                                                const R isig[4]) {
@@ -417,9 +472,14 @@ __device__ __forceinline__ void normal_eq_wide(const PmParams& P, WideSmem<R, G>
   }
   double* red = &sm.red[slot][0][0];
   double* mine = red + warp * RED;
-  ne_reduce_chunk<R, KT, 0>(mine, lane, d, cw, rw);
-  if constexpr (NCH > 1) ne_reduce_chunk<R, KT, 1>(mine, lane, d, cw, rw);
-  if constexpr (NCH > 2) ne_reduce_chunk<R, KT, 2>(mine, lane, d, cw, rw);
+  if constexpr (sizeof(R) == 4 && !MAC) {
+    static_assert(kLaneStatePad == kRow, "a warp's synthesis states hold the transposed entries");
+    ne_warp_sums<KT, 0>(lane, d, cw, rw, sm.ls[32 * warp], mine);
+  } else {
+    ne_reduce_chunk<R, KT, 0>(mine, lane, d, cw, rw);
+    if constexpr (NCH > 1) ne_reduce_chunk<R, KT, 1>(mine, lane, d, cw, rw);
+    if constexpr (NCH > 2) ne_reduce_chunk<R, KT, 2>(mine, lane, d, cw, rw);
+  }
   __syncthreads();
   for (int e = threadIdx.x; e < KT * KT + KT; e += 32 * G) {
     int idx;
@@ -465,7 +525,17 @@ __device__ __forceinline__ void rf_and_normal_eq_wide(const PmParams& P, WideSme
 #pragma unroll
       for (int s = 0; s < 4; ++s) d[r][s] = 0;
     }
-  normal_eq_wide<R, KT, G>(P, sm, slot, d, S, O, isig);
+  normal_eq_wide<R, KT, G, MAC>(P, sm, slot, d, S, O, isig);
+}
+
+// A condition that all lanes of a warp agree on, marked so (uniform): shuffles and
+// barriers behind such a branch need no convergence code.  The instances with a v_mac
+// row are compiled without the mark, which changed how the compiler fuses their
+// products and with it their last bits.
+template <bool MAC>
+__device__ __forceinline__ bool one_way(bool c) {
+  if constexpr (MAC) return c;
+  else return uniform(c);
 }
 
 // lm_mils over pixels of a wide grid: the control flow of invert_pixel with
@@ -473,12 +543,15 @@ __device__ __forceinline__ void rf_and_normal_eq_wide(const PmParams& P, WideSme
 // ZM: the line is a Zeeman multiplet (a separate instance, as in the one-warp
 // kernel); MAC: the grid has a v_mac row (dynamic shared memory holds MacSmem);
 // PIXGRID: every pixel has its own wavelengths (io.lambda_pix).
+// Bound by the barriers at which G - 1 warps wait for warp 0's solve and by issue:
+// marked branches and the normal equations' sums through shared memory took 65,536
+// pixels of 112 wavelengths from 28.3 to 27.0 ms and 3,000 of 33 from 1.32 to 1.25 ms.
 template <typename R, int KT, int G, int MINB, bool ZM, bool MAC, bool PIXGRID>
 __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_constant__ PmParams P,
                                                                      const PmIO io) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WideSmem<R, G>& sm = *reinterpret_cast<WideSmem<R, G>*>(smem_raw);
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int t = threadIdx.x, lane = t & 31, warp = MAC ? t >> 5 : __shfl_sync(kFull, t >> 5, 0);
   const bool valid = t < P.nl;
   double dl_t = P.dl[valid ? t : 0];
   const R omw_t = valid ? omw<R>(P, t) : R(0);
@@ -491,7 +564,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
     if (t == 0) sm.pix = atomicAdd(&io.ctr[PMC_NEXT], 1ull);
     __syncthreads();
     const unsigned long long pix = sm.pix;
-    if (pix >= (unsigned long long)io.npix) break;
+    if (one_way<MAC>(pix >= (unsigned long long)io.npix)) break;
     // the pixel's own wavelengths (the PSF taps stay the context's)
     const double* lp = PIXGRID ? io.lambda_pix + size_t(pix) * P.nl : nullptr;
     if constexpr (PIXGRID) dl_t = lp[valid ? t : 0] - P.lambda0;
@@ -515,7 +588,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
     int status = PM_PIX_MAXITER, iter = 0, accepted = 0, fallbacks = 0;
     double ochi = 0;
     R S[4];
-    if (nfree == 0) {
+    if (one_way<MAC>(nfree == 0)) {
       status = PM_PIX_NFREE;
       iter = -1;
 #pragma unroll
@@ -529,13 +602,13 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
       __syncthreads();
       bool stop = false, first = true;
       while (true) {
-        if (!first) {
+        if (one_way<MAC>(!first)) {
           if (warp == 0) {
             double dlt[KT];
             bool ok = true;
             double* scratch = reinterpret_cast<double*>(&sm.rf[0][0]);  // idle during the solve
             if (P.solver == PM_SOLVE_CHOLESKY) ok = solve_cholesky<KT>(sm.sv, scratch, lane, flambda, dlt);
-            if (P.solver != PM_SOLVE_CHOLESKY || !ok) {
+            if (P.solver != PM_SOLVE_CHOLESKY || one_way<MAC>(!ok)) {
               if (P.solver == PM_SOLVE_CHOLESKY) ++fallbacks;
               solve_eigen<KT>(sm.sv, scratch, lane, flambda);
 #pragma unroll
@@ -565,7 +638,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
           }
           accept = chi - ochi < 0.;
         }
-        if (accept) {
+        if (one_way<MAC>(accept)) {
           if (!first) flambda = flambda / (5.0 * factor);
           if (t < 11) m[t] = trial[t];
           // the filling-factor row: unmixed synthesis first, mixed after a step
@@ -588,7 +661,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
           }
           ++iter;
           if (P.logclambda) factor = double(log10f(float(chi)) / log10f(float(chi0)));
-          if (!(iter < P.miter && !stop)) break;  // lm_mils' do-while: at least one step
+          if (one_way<MAC>(!(iter < P.miter && !stop))) break;  // lm_mils' do-while: at least one step
         }
         first = false;
       }

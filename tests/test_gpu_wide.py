@@ -16,6 +16,7 @@ import pmilos_b200 as pm
 import pyoracle as po
 from conftest import GOLDEN
 from gpu_common import NOISE64, assert_plain_parity, reference_fast, within_tolerance
+from pmilos_b200 import workloads
 
 pytestmark = pytest.mark.gpu
 
@@ -203,3 +204,36 @@ def test_host_buffers_in_many_chunks_equal_one_call(monkeypatch):
         assert np.array_equal(many[k], one[k]), k
         assert np.array_equal(dev[k].cpu().numpy(), one[k]), k
     assert st["pixels"] == 600 and st["iterations"] == int(np.maximum(many["iters"], 0).sum())
+
+
+@pytest.mark.parametrize("nl,nterms", [(33, 9), (64, 10), (65, 9), (97, 10), (128, 9)])
+def test_fp32_wide_first_step_matches_fp64(nl, nterms):
+    """One LM step in FP32 and in FP64 at the edges of two and four warps, so that each
+    entry of the normal equations and each warp's share of it counts.
+
+    The step is measured in the response functions' norms (the square roots of the
+    normal matrix' diagonal).  So scaled, the matrix damped by lambda = 1 has
+    eigenvalues between 1 and nterms + 1: its inverse passes the entries' relative
+    error on at most about nterms + 1 times.  The FP32 response functions, whose error
+    rules, stay within 1e-3 of a row's norm or so, which gives 1e-2; the bound is 5e-2.
+    A lost entry or warp changes the step by a good part of itself.
+    """
+    w = workloads.config(2 if nterms == 10 else 1, npix=200)
+    offs = (np.arange(nl) - nl // 2) * (45.0 * 32 / nl)
+    w.offs, w.lam = offs, w.line.lambda0 + offs / 1000.0
+    w.psf = pm.psf_gaussian(60.0, w.lam)
+    w.nterms = nterms
+    obs = workloads.synthesize(w, rng=np.random.default_rng(nl))
+    sl = None if w.slight is None else np.asarray(w.slight, dtype=np.float32)
+    step, guess = [], np.asarray(w.guess, dtype=np.float64)
+    for precision in (pm.PREC_FP32, pm.PREC_FP64):
+        with pm.Inverter(w.line, w.lam, w.psf, noise=NOISE64, fix=w.fix, nterms=nterms, miter=1, ilambda=1.0,
+                         toplim=0.0, precision=precision, solver=pm.SOLVE_CHOLESKY) as inv:
+            step.append(np.asarray(inv.invert(obs, w.guess, slight=sl)["models"]) - guess)
+            rf = np.asarray(inv.synth(guess[None], rf=True, slight=sl)[1])[0]
+    norm = np.sqrt((rf.astype(np.float64) ** 2).sum(axis=(0, 2)))  # one per row
+    rows = [0, 1, 2, 3, 4, 5, 6, 7, 8, 10][:nterms]                # row 9 is the filling factor
+    a, b = (np.linalg.norm(s[:, rows] * norm, axis=1) for s in (step[0] - step[1], step[1]))
+    taken = b > 0
+    assert taken.mean() > 0.5
+    assert (a[taken] <= 5e-2 * b[taken]).mean() >= 0.95
