@@ -527,13 +527,17 @@ __device__ __forceinline__ void mac_triple(const PmParams& P, double k, int lane
   }
 }
 
-// The kernel of v_mac (and its derivative with DERIV) into xs; tr is scratch.
+// The kernel of v_mac (and its derivative with DERIV) into xs.  Scratch: tr or, where
+// tr holds the synthesis states, the part of xs that the kernel goes to.
 template <typename R, bool DERIV, typename SM>
 __device__ __forceinline__ void mac_prepare(const PmParams& P, SM& sm, double mac, double dl, int lane,
                                             bool valid) {
   double g, gd;
-  mac_kernel<DERIV>(P, mac, dl, lane, valid, reinterpret_cast<double*>(sm.tr), g, gd);
   R* xf = &sm.xs[0][0];
+  static_assert((4 * XSR - kMacK) * sizeof(R) >= 2 * NL * sizeof(double) && kMacK * sizeof(R) % sizeof(double) == 0,
+                "scratch for the kernel");
+  double* scratch = reinterpret_cast<double*>(SM::kSharedRows ? xf + kMacK : sm.tr);
+  mac_kernel<DERIV>(P, mac, dl, lane, valid, scratch, g, gd);
   mac_triple<R>(P, g, lane, xf + kMacK);
   if (DERIV) mac_triple<R>(P, gd, lane, xf + kMacD);
   if (lane == 0) sm.xs_dirty = 1;

@@ -35,22 +35,15 @@ struct alignas(16) PairBlock {
 // and scratch of the solvers and of the reductions); ls: the synthesis state that
 // the response functions are formed from, per lane; xs: padded Stokes rows of the
 // synthesis correlation.  The response functions overwrite the states (every lane
-// has its own in registers by then), except in the kernels with a macroturbulence
-// branch (APART), which use tr before.
-struct RowsShared {
+// has its own in registers by then); the macroturbulence kernel is formed in xs, so
+// that its instances share the rows too (16 warps per SM fit where 12 did: 16,384
+// pixels, 11 parameters: 7.63 -> 7.12 ms).
+struct alignas(16) RowsSmem {
   static constexpr bool kSharedRows = true;
   union {
     float tr[NL * kRow];
     float ls[NL][kLaneStatePad];
   };
-};
-struct RowsApart {
-  static constexpr bool kSharedRows = false;
-  float tr[NL * kRow];
-  float ls[NL][kLaneStatePad];
-};
-template <bool APART>
-struct alignas(16) RowsSmem : std::conditional_t<APART, RowsApart, RowsShared> {
   float xs[4][XSR];
   int xs_dirty;  // xs holds macroturbulence data: restore its zero padding before psf_rows
   int grid_cur;  // the grid whose padding xs has
@@ -485,13 +478,13 @@ __device__ __forceinline__ void pair_response(const PmParams& P, const PairBlock
                                               const ModelTerms<float>& mt, int lane, bool valid, double mac, double dl,
                                               float (&dmac)[4]) {
   const bool mac_on = MAC && uniform(mac > kMacMin);
-  if (mac_on) mac_prepare<float, true>(P, sm, mac, dl, lane, valid);  // before tr fills up
+  if (mac_on) mac_prepare<float, true>(P, sm, mac, dl, lane, valid);
   {
     ModelTerms<float> T;
     copy16(T, mt);
     LaneState<float> st;
     copy16(st, *reinterpret_cast<const LaneState<float>*>(sm.ls[lane]));
-    if constexpr (SM::kSharedRows) __syncwarp();  // the profiles overwrite the lanes' states
+    __syncwarp();  // the profiles overwrite the lanes' states
     rf_rows(P, T, st, sm.tr + lane);
   }
   if (mac_on) {
@@ -531,8 +524,8 @@ struct alignas(16) PixelSlot {
   long long job_k;
 };
 
-template <int KT, bool MAC>
-struct alignas(16) PairSmem : RowsSmem<MAC> {
+template <int KT>
+struct alignas(16) PairSmem : RowsSmem {
   PixelSlot<KT> px[2];
 };
 
@@ -909,7 +902,7 @@ __global__ void __launch_bounds__(128, MINB) invert_pair_kernel(
     const __grid_constant__ GridParams<MULTI ? PMK_MAX_GRIDS : 1> GS, const PmStreamIO sio) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NG = MULTI ? PMK_MAX_GRIDS : 1;
-  using SM = PairSmem<KT, MAC>;
+  using SM = PairSmem<KT>;
   const int lane = threadIdx.x & 31, warp = __shfl_sync(kFull, int(threadIdx.x >> 5), 0);
   const int half = lane >> 4;
   PairBlock* bs = reinterpret_cast<PairBlock*>(smem_raw);
@@ -1046,7 +1039,7 @@ int launch_invert_pair_inst(const PmGridSet& GS, const PmStreamIO& sio, cudaStre
   if (wpb > 4) wpb = 4;
   const int threads = 32 * wpb;
   constexpr int NG = MULTI ? PMK_MAX_GRIDS : 1;
-  using SM = PairSmem<KT, MAC>;
+  using SM = PairSmem<KT>;
   static_assert(sizeof(PairBlock) % 16 == 0 && sizeof(PixelSlot<KT>) % 16 == 0 && sizeof(SM) % 16 == 0 &&
                     sizeof(SolveSmem) <= 4 * XSR * sizeof(float) &&
                     eigen_scratch_doubles<KT>() * sizeof(double) <= NL * kRow * sizeof(float) &&
@@ -1078,7 +1071,7 @@ int launch_invert_pair_inst(const PmGridSet& GS, const PmStreamIO& sio, cudaStre
 // 20 warps per SM (96 registers, a few spills) hide more latency than 16 (128) where
 // there are pixels for them: nine parameters, 65,536 pixels: 8.57 ms against 8.91.
 // With more parameters the spills cost more than that (10 parameters 13.54 against
-// 13.33 ms, 11 with macroturbulence 8.56 against 8.00), and a call that does not
+// 13.33 ms, 11 with macroturbulence, 16,384 pixels: 8.06 against 7.09), and a call that does not
 // fill 16 warps per SM gains nothing by them.
 template <int KT, bool MULTI, bool MAC, bool PIXGRID = false>
 int launch_invert_pair(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t st, int num_sms, size_t* smem_out,

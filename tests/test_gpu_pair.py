@@ -38,7 +38,7 @@ def _inverter(w, solver=pm.SOLVE_DEFAULT):
 
 
 @pytest.mark.parametrize("npix", [1, 2, 3, 7, 9, 300])
-@pytest.mark.parametrize("nl,nterms", [(2, 9), (5, 9), (29, 10), (31, 11), (32, 9)])
+@pytest.mark.parametrize("nl,nterms", [(2, 9), (5, 9), (29, 10), (3, 11), (31, 11), (32, 11), (32, 9)])
 def test_a_pixel_alone_equals_the_pixel_in_a_call(nl, nterms, npix):
     w, obs = _cube(nl, nterms, npix)
     if npix > 2:
