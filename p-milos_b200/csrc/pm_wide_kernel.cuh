@@ -451,10 +451,10 @@ __device__ __forceinline__ void ne_warp_sums(int lane, const float (&d)[KT][4], 
 }
 
 // Normal equations over the block: packed entries reduced per warp (in FP32 through
-// the warp's synthesis states, which the response functions have read; in FP64 and
-// with a v_mac row as normal_eq), then the G warp totals summed in warp order into
-// sv.ab.
-template <typename R, int KT, int G, bool MAC>
+// the warp's synthesis states, which the response functions have read; in FP64, for
+// multiplets and with a v_mac row as normal_eq), then the G warp totals summed in warp
+// order into sv.ab.
+template <typename R, int KT, int G, bool MAC, bool ZM>
 __device__ __forceinline__ void normal_eq_wide(const PmParams& P, WideSmem<R, G>& sm, int& slot,
                                                const R (&d)[KT][4], const R S[4], const float O[4],
                                                const R isig[4]) {
@@ -472,7 +472,7 @@ __device__ __forceinline__ void normal_eq_wide(const PmParams& P, WideSmem<R, G>
   }
   double* red = &sm.red[slot][0][0];
   double* mine = red + warp * RED;
-  if constexpr (sizeof(R) == 4 && !MAC) {
+  if constexpr (sizeof(R) == 4 && !MAC && !ZM) {
     static_assert(kLaneStatePad == kRow, "a warp's synthesis states hold the transposed entries");
     ne_warp_sums<KT, 0>(lane, d, cw, rw, sm.ls[32 * warp], mine);
   } else {
@@ -525,16 +525,17 @@ __device__ __forceinline__ void rf_and_normal_eq_wide(const PmParams& P, WideSme
 #pragma unroll
       for (int s = 0; s < 4; ++s) d[r][s] = 0;
     }
-  normal_eq_wide<R, KT, G, MAC>(P, sm, slot, d, S, O, isig);
+  normal_eq_wide<R, KT, G, MAC, ZM>(P, sm, slot, d, S, O, isig);
 }
 
 // A condition that all lanes of a warp agree on, marked so (uniform): shuffles and
-// barriers behind such a branch need no convergence code.  The instances with a v_mac
-// row are compiled without the mark, which changed how the compiler fuses their
-// products and with it their last bits.
-template <bool MAC>
+// barriers behind such a branch need no convergence code.  The instances of
+// multiplets and those with a v_mac row are compiled without the mark, which changed
+// how the compiler fuses their products and with it their last bits and, here and
+// there, the iteration counts.
+template <bool PLAIN>
 __device__ __forceinline__ bool one_way(bool c) {
-  if constexpr (MAC) return c;
+  if constexpr (PLAIN) return c;
   else return uniform(c);
 }
 
@@ -551,7 +552,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
                                                                      const PmIO io) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   WideSmem<R, G>& sm = *reinterpret_cast<WideSmem<R, G>*>(smem_raw);
-  const int t = threadIdx.x, lane = t & 31, warp = MAC ? t >> 5 : __shfl_sync(kFull, t >> 5, 0);
+  const int t = threadIdx.x, lane = t & 31, warp = MAC || ZM ? t >> 5 : __shfl_sync(kFull, t >> 5, 0);
   const bool valid = t < P.nl;
   double dl_t = P.dl[valid ? t : 0];
   const R omw_t = valid ? omw<R>(P, t) : R(0);
@@ -564,7 +565,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
     if (t == 0) sm.pix = atomicAdd(&io.ctr[PMC_NEXT], 1ull);
     __syncthreads();
     const unsigned long long pix = sm.pix;
-    if (one_way<MAC>(pix >= (unsigned long long)io.npix)) break;
+    if (one_way<MAC || ZM>(pix >= (unsigned long long)io.npix)) break;
     // the pixel's own wavelengths (the PSF taps stay the context's)
     const double* lp = PIXGRID ? io.lambda_pix + size_t(pix) * P.nl : nullptr;
     if constexpr (PIXGRID) dl_t = lp[valid ? t : 0] - P.lambda0;
@@ -588,7 +589,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
     int status = PM_PIX_MAXITER, iter = 0, accepted = 0, fallbacks = 0;
     double ochi = 0;
     R S[4];
-    if (one_way<MAC>(nfree == 0)) {
+    if (one_way<MAC || ZM>(nfree == 0)) {
       status = PM_PIX_NFREE;
       iter = -1;
 #pragma unroll
@@ -602,13 +603,13 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
       __syncthreads();
       bool stop = false, first = true;
       while (true) {
-        if (one_way<MAC>(!first)) {
+        if (one_way<MAC || ZM>(!first)) {
           if (warp == 0) {
             double dlt[KT];
             bool ok = true;
             double* scratch = reinterpret_cast<double*>(&sm.rf[0][0]);  // idle during the solve
             if (P.solver == PM_SOLVE_CHOLESKY) ok = solve_cholesky<KT>(sm.sv, scratch, lane, flambda, dlt);
-            if (P.solver != PM_SOLVE_CHOLESKY || one_way<MAC>(!ok)) {
+            if (P.solver != PM_SOLVE_CHOLESKY || one_way<MAC || ZM>(!ok)) {
               if (P.solver == PM_SOLVE_CHOLESKY) ++fallbacks;
               solve_eigen<KT>(sm.sv, scratch, lane, flambda);
 #pragma unroll
@@ -638,7 +639,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
           }
           accept = chi - ochi < 0.;
         }
-        if (one_way<MAC>(accept)) {
+        if (one_way<MAC || ZM>(accept)) {
           if (!first) flambda = flambda / (5.0 * factor);
           if (t < 11) m[t] = trial[t];
           // the filling-factor row: unmixed synthesis first, mixed after a step
@@ -661,7 +662,7 @@ __global__ void __launch_bounds__(32 * G, MINB) invert_wide_kernel(const __grid_
           }
           ++iter;
           if (P.logclambda) factor = double(log10f(float(chi)) / log10f(float(chi0)));
-          if (one_way<MAC>(!(iter < P.miter && !stop))) break;  // lm_mils' do-while: at least one step
+          if (one_way<MAC || ZM>(!(iter < P.miter && !stop))) break;  // lm_mils' do-while: at least one step
         }
         first = false;
       }
