@@ -591,21 +591,12 @@ __device__ __forceinline__ void xs_restore(SM& sm, int lane) {
   __syncwarp();
 }
 
-// Synthesis of the model at this lane's wavelength, PSF (or macroturbulence)
-// and stray light included.  S gets the final (mixed) profile, Su the profile
-// before the stray-light mix.  The per-model terms and this lane's synthesis
-// state are left in shared memory for the response functions, as the reference
-// leaves them in globals.  MAC: the kernel has a v_mac response row (NTERMS >=
-// 10), so v_mac may be nonzero.  dl: this lane's wavelength offset lambda -
-// lambda0 (the grid's, or the pixel's own).
-template <typename R, bool MAC, bool SL, typename SM, typename Lane, typename Psf>
-__device__ __forceinline__ void synthesize_terms(const PmParams& P, SM& sm, const ModelTerms<R>& T, double mac,
+// The PSF (psf) or macroturbulence correlation of the synthesized profiles S and the
+// stray-light mix; Su: the profiles before the mix.  SL: compiled with the mix.
+template <typename R, bool MAC, bool SL, typename SM, typename Psf>
+__device__ __forceinline__ void convolve_and_mix(const PmParams& P, SM& sm, const ModelTerms<R>& T, double mac,
                                                  const float* sl_pix, int lane, bool valid, double dl, R S[4],
-                                                 R Su[4], Lane synth, Psf psf) {
-  R s0[4];
-  synth(s0);
-#pragma unroll
-  for (int s = 0; s < 4; ++s) S[s] = s0[s];
+                                                 R Su[4], Psf psf) {
   if (MAC && mac > kMacMin) {
     R* xf = &sm.xs[0][0];
 #pragma unroll
@@ -633,17 +624,26 @@ __device__ __forceinline__ void synthesize_terms(const PmParams& P, SM& sm, cons
   __syncwarp();
 }
 
+// Synthesis of the model at this lane's wavelength, PSF (or macroturbulence)
+// and stray light included.  S gets the final (mixed) profile, Su the profile
+// before the stray-light mix.  The per-model terms and this lane's synthesis
+// state are left in shared memory for the response functions, as the reference
+// leaves them in globals.  MAC: the kernel has a v_mac response row (NTERMS >=
+// 10), so v_mac may be nonzero.  dl: this lane's wavelength offset lambda -
+// lambda0 (the grid's, or the pixel's own).
+// The multiplet instances' last bits hang on this form: with the synthesis behind a
+// function argument the compiler fused other products.
 template <typename R, bool MAC, bool ZM, typename SM>
 __device__ __forceinline__ void synthesize(const PmParams& P, SM& sm, const double* m,
                                            const float* sl_pix, int lane, bool valid, double dl, R S[4], R Su[4]) {
   ModelTerms<R> T;
+  LaneState<R> st;
   model_terms<R, ZM>(P, m, T);
-  synthesize_terms<R, MAC, true>(P, sm, T, MAC ? m[9] : 0.0, sl_pix, lane, valid, dl, S, Su, [&](R(&out)[4]) {
-    LaneState<R> st;
-    synth_lane<R, ZM>(P, T, dl, st, out);
-    copy16(*reinterpret_cast<LaneState<R>*>(sm.ls[lane]), st);
-    if (lane == 0) copy16(sm.mt, T);
-  }, [&] { psf_rows<R>(P, sm, lane, valid, S); });
+  synth_lane<R, ZM>(P, T, dl, st, S);
+  copy16(*reinterpret_cast<LaneState<R>*>(sm.ls[lane]), st);
+  if (lane == 0) copy16(sm.mt, T);
+  convolve_and_mix<R, MAC, true>(P, sm, T, MAC ? m[9] : 0.0, sl_pix, lane, valid, dl, S, Su,
+                                 [&] { psf_rows<R>(P, sm, lane, valid, S); });
 }
 
 template <typename R, typename SM>

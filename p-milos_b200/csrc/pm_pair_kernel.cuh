@@ -713,8 +713,8 @@ __device__ __forceinline__ void pair_pass(const PmParams& P, const PairBlock& bs
   {
     ModelTerms<float> T;
     copy16(T, px.mt);
-    synthesize_terms<float, MAC, (KT >= 10)>(P, sm, T, mac, sl, lane, valid, dl, S, Su,
-                                             [&](float(&out)[4]) { pair_synth(P, T, dl, sm.ls[lane], out); },
+    pair_synth(P, T, dl, sm.ls[lane], S);
+    convolve_and_mix<float, MAC, (KT >= 10)>(P, sm, T, mac, sl, lane, valid, dl, S, Su,
                                              [&] { pair_psf(P, bs, sm, lane, valid, S); });
   }
 #pragma unroll

@@ -48,3 +48,33 @@ def _inverted_as_recorded(file, name):
 @pytest.mark.parametrize("name", ["nine_33", "stray_97", "stray_97_grids", "stray_64_grids"])
 def test_wide_grids(name):
     _inverted_as_recorded("wide_multiplet_results.npz", name)
+
+
+@pytest.mark.parametrize("name", ["mac_15", "mac_30_grids"])
+def test_one_warp_grids_with_a_v_mac_row(name):
+    _inverted_as_recorded("multiplet_results.npz", name)
+
+
+def test_served_grids_with_a_v_mac_row():
+    """The persistent kernel's instance for several grids."""
+    cases = [_case("multiplet_results.npz", f"served_{i}") for i in range(2)]
+    grids = [pm.Grid(lam=d["lam"], psf=d["psf"], guess=d["guess"], noise=NOISE64, fix=list(d["fix"]), nterms=11,
+                     miter=30) for d, _ in cases]
+    with pm.Server(pm.LineData(*LINE), grids, hbm_budget_bytes=1 << 26) as srv:
+        for i, (d, _) in enumerate(cases):
+            srv.set_slight(i, d["slight"])
+        ids = [srv.submit(i, d["obs"]) for i, (d, _) in enumerate(cases)]
+        for (_, want), sid in zip(cases, ids):
+            r = srv.wait(sid)
+            for k in want:
+                assert np.array_equal(r[k], want[k]), k
+
+
+@pytest.mark.parametrize("name", ["synth64_10a", "synth64_10m", "synth64_11"])
+def test_fp64_synthesis(name):
+    """Profiles and response functions with stray light or a v_mac row."""
+    d, want = _case("multiplet_results.npz", name)
+    with _inverter(d, pm.PREC_FP64) as inv:
+        spectra, rf = inv.synth(d["models"], rf=True, slight=d.get("slight"))
+    assert np.array_equal(spectra, want["spectra"])
+    assert np.array_equal(rf, want["rf"])
