@@ -894,8 +894,9 @@ __device__ __forceinline__ void pair_end(const PmParams& P, PixelSlot<KT>& px, i
 // a round, so that the warps of a launch share a small call's pixels evenly) and
 // owns it: the pixel starts once the ticket is published.  While the other slot
 // holds a pixel the warp goes on with it; with nothing to do it sleeps between
-// looks at the queue, up to the wait limit (then PMQ_ERR_WAIT), and ends once the
-// queue is closed and its tickets are beyond the final count.  MULTI: the launch
+// looks at the queue, up to the wait limit after the last publication it saw (then
+// PMQ_ERR_WAIT: its own tickets may be far ahead of a slow producer's), and ends once
+// the queue is closed and its tickets are beyond the final count.  MULTI: the launch
 // serves up to PMK_MAX_GRIDS grids (a server's), each pixel on its own.
 template <int KT, int MINB, bool MULTI, bool MAC, bool PIXGRID>
 __global__ void __launch_bounds__(128, MINB) invert_pair_kernel(
@@ -934,7 +935,9 @@ __global__ void __launch_bounds__(128, MINB) invert_pair_kernel(
       if (!closed && __ballot_sync(kFull, waiting && (unsigned long long)held >= avail) && (active == 0 || ++age >= 4)) {
         age = 0;
         closed = ld_acquire(&sio.q->closed) != 0;  // written after the last publication
-        avail = ld_acquire(&sio.q->avail);
+        const unsigned long long seen = ld_acquire(&sio.q->avail);
+        if (uniform(seen != avail)) since = -1;
+        avail = seen;
       }
       bool start = false, end = false;
       if (waiting && (unsigned long long)held < avail) {
@@ -981,7 +984,11 @@ __global__ void __launch_bounds__(128, MINB) invert_pair_kernel(
       }
       if (active == 0) {
         if (drained == 3u) break;
-        if (started) continue;
+        if (started) {
+          since = -1;
+          sleep_ns = 32;
+          continue;
+        }
         const long long now = global_ns();
         if (since < 0) since = now;
         if (uniform(now - since > sio.wait_limit_ns)) {

@@ -102,7 +102,7 @@ struct PmStreamIO {
   int max_pixels;           // no more pixels than this will be published (0: not known): no more warps are launched
   long long first_job;      // no ticket left belongs to a job before this one
   long long published;      // every ticket, when all were published and the queue closed before the launch; else 0
-  long long wait_limit_ns;  // longest wait for a ticket before giving up with PMQ_ERR_WAIT
+  long long wait_limit_ns;  // longest wait without a publication before giving up with PMQ_ERR_WAIT
 };
 
 struct PmIO {

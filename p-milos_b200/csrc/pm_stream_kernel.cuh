@@ -16,8 +16,9 @@ namespace {
 // if it is not yet published, the warp waits for its publication, so a ticket
 // is never handed out twice nor lost.  The kernel ends when the host closes the
 // queue (PmStreamQ::closed, written after the last publication): warps holding
-// tickets beyond the final count exit.  Waits are bounded: after wait_limit_ns
-// without its ticket a warp sets PMQ_ERR_WAIT and exits.
+// tickets beyond the final count exit.  Waits are bounded: a waiting warp that sees no
+// publication for wait_limit_ns sets PMQ_ERR_WAIT and exits.  (The limit does not
+// count from the warp's own ticket: a slow producer may take longer to reach it.)
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
   unsigned long long v;
@@ -35,9 +36,13 @@ __device__ __forceinline__ long long global_ns() {
 __device__ long long next_ticket(PmStreamQ* q, long long limit_ns) {
   const unsigned long long t = atomicAdd(&q->next, 1ull);
   long long since = -1;
+  unsigned long long avail = 0;
   unsigned sleep = 32;
   while (true) {
-    if (t < ld_acquire(&q->avail)) return (long long)t;
+    const unsigned long long seen = ld_acquire(&q->avail);
+    if (t < seen) return (long long)t;
+    if (seen != avail) since = -1;
+    avail = seen;
     if (ld_acquire(&q->closed)) {
       // closed is written after the last publication: one more look
       return t < ld_acquire(&q->avail) ? (long long)t : -1;
