@@ -381,9 +381,10 @@ int pm_set_tuning(pm_ctx *ctx, const pm_tuning *in);
 /* Autotuner: inverts npix sample pixels (host buffers, the same call path as
  * pm_invert_batch with PM_MEM_HOST, so copies and kernel are both timed) once per
  * candidate tuning and repetition, and keeps the fastest tuning in the context.
- * Candidates: variants 0 and 1 with warps_per_block {1, 2, 4}, variant 2 with
- * {8, 16}, each with staging_depth {0, 2, 4}.  *out (nullable) receives the
- * choice.  No counterpart in the reference. */
+ * Candidates on one-warp grids: warps_per_block {1, 2, 4} with staging_depth
+ * {0, 2, 4}, as variant 1; on wider grids, which have one launch, the context's
+ * tuning with staging_depth 0.  *out (nullable) receives the choice.  No
+ * counterpart in the reference. */
 int pm_autotune(pm_ctx *ctx, int64_t npix, const float *spectro, const float *slight, int slight_mode,
                 const pm_model *guess, int reps, pm_tuning *out);
 

@@ -1264,17 +1264,15 @@ extern "C" int pm_autotune(pm_ctx* c, int64_t npix, const float* spectro, const 
   pm_model* models = static_cast<pm_model*>(out_buf.p);
   float* chi = reinterpret_cast<float*>(models + npix);
   int* its = reinterpret_cast<int*>(chi + npix);
+  // one candidate for each launch that differs: one-warp grids run the same kernel
+  // whatever the variant, in blocks of at most four warps; multi-warp grids are not
+  // streamed and have one block size
   std::vector<pm_tuning> cands;
-  const bool fp32 = c->precision == PM_PREC_FP32;
-  for (int variant : {0, 1, 2}) {
-    if (!fp32 && variant != c->tuning.variant) continue;  // the FP64 kernel has one register budget
-    for (int wpb : {1, 2, 4, 8, 16}) {
-      if ((variant == 2) != (wpb >= 8)) continue;  // the block sizes of each variant
-      for (int depth : {0, 2, 4}) {
-        if (c->P.G != 1 && depth != 0) continue;  // multi-warp grids are not streamed
-        cands.push_back(pm_tuning{variant, depth, wpb, c->tuning.graphs});
-      }
-    }
+  if (c->P.G != 1) {
+    cands.push_back(pm_tuning{c->tuning.variant, 0, c->tuning.warps_per_block, c->tuning.graphs});
+  } else {
+    for (int wpb : {1, 2, 4})
+      for (int depth : {0, 2, 4}) cands.push_back(pm_tuning{1, depth, wpb, c->tuning.graphs});
   }
   const pm_tuning saved = c->tuning;
   pm_tuning best = saved;
