@@ -898,8 +898,8 @@ __device__ __forceinline__ void pair_end(const PmParams& P, PixelSlot<KT>& px, i
 // PMQ_ERR_WAIT: its own tickets may be far ahead of a slow producer's), and ends once
 // the queue is closed and its tickets are beyond the final count.  MULTI: the launch
 // serves up to PMK_MAX_GRIDS grids (a server's), each pixel on its own.
-template <int KT, int MINB, bool MULTI, bool MAC, bool PIXGRID>
-__global__ void __launch_bounds__(128, MINB) invert_pair_kernel(
+template <int KT, bool MULTI, bool MAC, bool PIXGRID>
+__global__ void __launch_bounds__(128, 4) invert_pair_kernel(
     const __grid_constant__ GridParams<MULTI ? PMK_MAX_GRIDS : 1> GS, const PmStreamIO sio) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   constexpr int NG = MULTI ? PMK_MAX_GRIDS : 1;
@@ -1040,8 +1040,13 @@ __global__ void __launch_bounds__(128, MINB) invert_pair_kernel(
   }
 }
 
-template <int KT, int MINB, bool MULTI, bool MAC, bool PIXGRID>
-int launch_invert_pair_inst(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t st, int num_sms, size_t* smem_out,
+// 16 warps per SM (128 registers).  20 (96 registers, spills) hide more latency and gain
+// up to 1% on large calls of nine parameters, but lose elsewhere: 65,536 pixels 7.80 ms
+// with 16, 7.78 with 20; 2,800 pixels 787, 851 us; 65,025 pixels of 15 wavelengths 6.73,
+// 7.00 ms; nine served scans of 10,000 pixels 13.9, 14.5 ms; 11 parameters, 16,384
+// pixels 7.16, 8.08 ms.
+template <int KT, bool MULTI, bool MAC, bool PIXGRID = false>
+int launch_invert_pair(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t st, int num_sms, size_t* smem_out,
                        int wpb, int reserve) {
   if (wpb > 4) wpb = 4;
   const int threads = 32 * wpb;
@@ -1055,7 +1060,7 @@ int launch_invert_pair_inst(const PmGridSet& GS, const PmStreamIO& sio, cudaStre
                 "pair shared-memory layout");
   const size_t smem = NG * sizeof(PairBlock) + sizeof(SM) * wpb;
   if (smem_out) *smem_out = smem;
-  auto kern = invert_pair_kernel<KT, MINB, MULTI, MAC, PIXGRID>;
+  auto kern = invert_pair_kernel<KT, MULTI, MAC, PIXGRID>;
   GridParams<NG> gp;  // copied into the launch
   gp.ngrids = GS.ngrids < NG ? GS.ngrids : NG;
   for (int g = 0; g < gp.ngrids; ++g) gp.g[g] = GS.g[g];
@@ -1066,28 +1071,13 @@ int launch_invert_pair_inst(const PmGridSet& GS, const PmStreamIO& sio, cudaStre
   if (e != cudaSuccess || per_sm < 1) return snprintf(pmk_g_err, sizeof pmk_g_err, "occupancy: %s", cudaGetErrorString(e)), PM_EIO;
   int blocks = per_sm * num_sms - reserve > 1 ? per_sm * num_sms - reserve : 1;
   // a call of few pixels: one per warp, and no warps that would only draw tickets
-  // beyond the last (one lm_mils call 233 -> 222 us, with the count known to the
-  // kernel as well)
+  // beyond the last (without the limit: 100 pixels from host arrays 509 us, with it 428;
+  // 592 on the device 564, 407; 1,800 on the device 666, 630; one lm_mils call the same)
   if (sio.max_pixels > 0 && blocks > (sio.max_pixels + wpb - 1) / wpb) blocks = (sio.max_pixels + wpb - 1) / wpb;
   kern<<<unsigned(blocks), threads, smem, st>>>(gp, sio);
   e = cudaGetLastError();
   if (e != cudaSuccess) return snprintf(pmk_g_err, sizeof pmk_g_err, "pair launch: %s", cudaGetErrorString(e)), PM_EIO;
   return PM_OK;
-}
-
-// 20 warps per SM (96 registers, a few spills) hide more latency than 16 (128) where
-// there are pixels for them: nine parameters, 65,536 pixels: 8.57 ms against 8.91.
-// With more parameters the spills cost more than that (10 parameters 13.54 against
-// 13.33 ms, 11 with macroturbulence, 16,384 pixels: 8.06 against 7.09), and a call that does not
-// fill 16 warps per SM gains nothing by them.
-template <int KT, bool MULTI, bool MAC, bool PIXGRID = false>
-int launch_invert_pair(const PmGridSet& GS, const PmStreamIO& sio, cudaStream_t st, int num_sms, size_t* smem_out,
-                       int wpb, int reserve) {
-  if constexpr (KT == 9) {
-    if (!(sio.max_pixels > 0 && sio.max_pixels <= 16 * num_sms))
-      return launch_invert_pair_inst<KT, 5, MULTI, MAC, PIXGRID>(GS, sio, st, num_sms, smem_out, wpb, reserve);
-  }
-  return launch_invert_pair_inst<KT, 4, MULTI, MAC, PIXGRID>(GS, sio, st, num_sms, smem_out, wpb, reserve);
 }
 
 }  // namespace

@@ -91,7 +91,7 @@ def test_served_scans_of_pixels_that_end_at_once():
             assert np.array_equal(r[part][k][~odd], r[full][k][~odd]), k
 
 
-@pytest.mark.parametrize("npix", [1500, 3000])  # up to 16 warps per SM, and beyond (nine parameters: another instance)
+@pytest.mark.parametrize("npix", [1500, 3000])  # a warp per pixel, and more pixels than warps
 @pytest.mark.parametrize("nterms", [9, 10])
 def test_every_launch_shape_gives_the_same_bits(nterms, npix):
     """Each variant and block size, with the pixel count published before the launch
