@@ -5,11 +5,12 @@
 // linkage.
 //
 // What bounds this path is instruction issue, and the issue rate is bound by the
-// instruction cache: straight-line code runs at 0.9 instructions per cycle and
-// scheduler up to 32 KB, at 0.3-0.5 beyond it.  So the LM loop is written for few
-// instructions and little code: the response functions, the correlation and the
-// factorisation are rolled loops, the sums of the normal equations go through
-// shared memory, and branches that the warp takes as one are marked so (uniform).
+// instruction cache: straight-line code, 16 warps at different places, runs at 0.96
+// instructions per cycle and scheduler up to 32 KB, at 0.87 at 36 KB, 0.6 at 40-48 KB
+// and 0.38 from 80 KB on.  So the LM loop is written for few instructions and little
+// code: the response functions, the correlation and the factorisation are rolled
+// loops, the sums of the normal equations go through shared memory, and branches that
+// the warp takes as one are marked so (uniform).
 #pragma once
 #include "pm_stream_kernel.cuh"
 
@@ -318,8 +319,10 @@ __device__ __forceinline__ void rf_rows(const PmParams& P, const ModelTerms<floa
 // PSF correlation of the 32 response-function profiles, one profile per lane
 // (me_der.c:471-496): out[k] = sum_m x[m] G[m - k + nl/2].  A loop over the inputs
 // m, four at a time: one load of the inputs from the lane's own row, and their taps
-// as one window of 35 consecutive entries of a reversed tap row (9 broadcast vector
-// loads for 128 products: in step, warps were bound by these loads).  Every
+// as one window of 35 consecutive entries of a reversed tap row, which is there twice,
+// once shifted by an entry, so that the pairs at odd offsets are aligned too: 18
+// broadcast vector loads for 128 products (the second row: 8.57 -> 8.41 ms for 65,536
+// pixels of the form of then; shared memory is the busiest pipe of this kernel).  Every
 // output adds its products in the order of m.  The last group's inputs beyond the
 // grid are zero.  Stokes-I rows correlate Ic - x with Ic = max of the row's end
 // points; the other rows run the same code with sign 1 and Ic = 0.

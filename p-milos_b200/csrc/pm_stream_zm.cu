@@ -2,9 +2,9 @@
 // N_SIG > 1, e.g. Fe I 6301.5, 5P2.0-5D2.0): the component loop of the synthesis
 // and the last component's derivative terms (ZM = true), on one grid, on a
 // server's several grids, or on per-pixel grids; with a v_mac row (MAC: NTERMS
-// 11, or 10 with the filling factor fixed) or without.  The launch shapes are
-// those of the triplet kernels: FP32 at 4 blocks per SM (128 registers), FP64
-// at 1.
+// 11, or 10 with the filling factor fixed) or without.  One pixel per warp: FP32
+// at 4 blocks per SM (128 registers), FP64 with one block's register budget
+// (triplets have kernels and shapes of their own: pm_pair_kernel.cuh, pm_stream.cu).
 #include "pm_stream_kernel.cuh"
 
 namespace {
